@@ -37,44 +37,44 @@ def listed() -> list[dict]:
     return [
         # one robot in a control or teleoperation loop: eight eager steps from
         # a given state, where launches and host work are what is waited for
-        dict(name="rollout 1 humanoid", kind="rollout", robot="humanoid", worlds=1, steps=8, precision="fp64",
+        dict(name="rollout-humanoid-1", kind="rollout", robot="humanoid", worlds=1, steps=8, precision="fp64",
              warm_start="previous_velocity", graph=False),
         # sampling or policy training: a batch of humanoids rolled out from
         # given states, two steps per captured graph, the fastest settings
-        dict(name="rollout 4096 humanoids", kind="rollout", robot="humanoid", worlds=4096, steps=8, precision="fp32",
+        dict(name="rollout-humanoid-4096", kind="rollout", robot="humanoid", worlds=4096, steps=8, precision="fp32",
              warm_start="learned", graph=True),
         # manipulation: an arm gripping one of eight stacked boxes, worlds of
         # several trees (tree-blocked layout), reference settings
-        dict(name="rollout 512 arms, 8 boxes", kind="rollout", robot="arm_boxes", boxes=8, worlds=512, steps=2,
+        dict(name="rollout-arm-boxes-512", kind="rollout", robot="arm_boxes", boxes=8, worlds=512, steps=2,
              precision="fp64", warm_start="previous_velocity", graph=False),
         # free motion and contact rows of the batch, as a program with a
         # solver of its own takes them
-        dict(name="rows 4096 humanoids", kind="rows", robot="humanoid", worlds=4096, precision="fp64",
+        dict(name="rows-humanoid-4096", kind="rows", robot="humanoid", worlds=4096, precision="fp64",
              point="contact_midpoint", weight="diag_delassus"),
         # the same on a small batch of another robot and in the other modes
-        dict(name="rows 250 quadrupeds", kind="rows", robot="quadruped", worlds=250, precision="fp64",
+        dict(name="rows-quadruped-250", kind="rows", robot="quadruped", worlds=250, precision="fp64",
              point="witness_point", weight="body_inertia"),
         # the contact solve alone: the reference's method on the headline batch
-        dict(name="solve 4096 x 35 fp64", kind="solve", dofs=35, contacts=32, worlds=4096, precision="fp64",
+        dict(name="solve-35x4096-fp64", kind="solve", dofs=35, contacts=32, worlds=4096, precision="fp64",
              line_search="armijo_decay"),
         # ... with the FP32 Hessian on quadrupeds, a batch size that is no
         # multiple of anything, the exact line search
-        dict(name="solve 3001 x 18 fp32", kind="solve", dofs=18, contacts=16, worlds=3001, precision="fp32",
+        dict(name="solve-18x3001-fp32", kind="solve", dofs=18, contacts=16, worlds=3001, precision="fp32",
              line_search="exact_root"),
         # ... on a robot without a specialised kernel
-        dict(name="solve 777 x 27 fp64", kind="solve", dofs=27, contacts=24, worlds=777, precision="fp64",
+        dict(name="solve-27x777-fp64", kind="solve", dofs=27, contacts=24, worlds=777, precision="fp64",
              line_search="monotone_decay"),
         # an uneven batch in one launch: arms with a box (13 DOFs), quadrupeds
         # (18) and humanoids (35), each world at its own DOF count
-        dict(name="solve 6000 uneven fp32", kind="uneven", worlds=6000, contacts=64, precision="fp32",
+        dict(name="solve-uneven-6000-fp32", kind="uneven", worlds=6000, contacts=64, precision="fp32",
              line_search="armijo_decay"),
         # clutter: worlds of 64 stacked free boxes, 384 DOFs, about 400 contacts
-        dict(name="solve 296 x 64 boxes fp32", kind="boxes", boxes=64, contacts=448, worlds=296, precision="fp32",
+        dict(name="solve-boxes64-296-fp32", kind="boxes", boxes=64, contacts=448, worlds=296, precision="fp32",
              line_search="armijo_decay"),
         # contacts of stacked boxes found anew from the pose
-        dict(name="contacts 256 x 64 boxes", kind="contacts", boxes=64, worlds=256),
+        dict(name="contacts-boxes64-256", kind="contacts", boxes=64, worlds=256),
         # training the warm-start network, at the batch its training uses
-        dict(name="train step 8192", kind="train", batch=8192),
+        dict(name="train-8192", kind="train", batch=8192),
     ]
 
 
