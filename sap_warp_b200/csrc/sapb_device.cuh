@@ -165,15 +165,20 @@ __device__ __forceinline__ void effective_pd_gains(double kp, double kd, double 
   }
 }
 
-// Reciprocal for pivots on a serial critical path.  Newton-Raphson iteration
-// for 1/d (x <- x + x (1 - d x), each step squaring the relative error) from
-// the FP32 reciprocal as seed: two steps take the ~2^-23 seed error to below
-// 2^-52, i.e. within an ulp or two of the correctly rounded quotient.  Values
-// outside the FP32 range (or not finite) use the IEEE division.
+// Reciprocal for pivots on a serial critical path: the hardware's approximate
+// FP64 reciprocal as seed, then two Newton-Raphson steps for 1/d (x <- x + x
+// (1 - d x), each squaring the relative error), which take the seed's ~1e-6
+// below 2^-52, within an ulp or two of the correctly rounded quotient.
+// Dependent latency measured on B200: 48 cycles, against 61 of a division
+// and 130 of a seed converted from the FP32 reciprocal and back (4096
+// 35-DOF FP64 solves 1278 -> 1195 us).  Magnitudes near the ends of the range
+// (where the seed or the residual leaves it) and values that are not finite
+// take the division.
 __device__ __forceinline__ double fast_recip(double d) {
   const double ad = fabs(d);
-  if (!(ad > 1.0e-30 && ad < 1.0e30)) return 1.0 / d;
-  double x = (double)__frcp_rn((float)d);
+  if (!(ad > 1.0e-290 && ad < 1.0e290)) return 1.0 / d;
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
   double e = fma(-d, x, 1.0);
   x = fma(x, e, x);
   e = fma(-d, x, 1.0);
