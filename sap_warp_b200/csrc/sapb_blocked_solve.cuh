@@ -149,6 +149,7 @@ using namespace blk;
 template <int NT, typename HT, int NB>
 struct BWorld {
   // -- the world interface of the line searches --
+  static constexpr int kCoefWarps = NT / 32;
   int count, n, C;
   double* vec;
   double* con;
@@ -162,17 +163,17 @@ struct BWorld {
     const int t = terms ? bterm(k) : -1;
     return vec + (size_t)(t >= 0 ? kBVecs + t : bslot(k)) * n;
   }
-  __device__ __forceinline__ double* Cn(int k) const { return con + (size_t)k * C; }
+  __device__ __forceinline__ double* cn(int c) const { return con + c * (int)C_END; }
   __device__ ContactConst cc(int c) const {
     ContactConst x;
-    x.rt = Cn(C_RT)[c];
-    x.rn = Cn(C_RN)[c];
-    x.rt_inv = Cn(C_RTINV)[c];
-    x.rn_inv = Cn(C_RNINV)[c];
-    x.vhat_n = Cn(C_VHAT)[c];
-    x.mu = Cn(C_MU)[c];
-    x.mu_hat = Cn(C_MUHAT)[c];
-    x.factor = Cn(C_FACTOR)[c];
+    x.rt = cn(c)[C_RT];
+    x.rn = cn(c)[C_RN];
+    x.rt_inv = cn(c)[C_RTINV];
+    x.rn_inv = cn(c)[C_RNINV];
+    x.vhat_n = cn(c)[C_VHAT];
+    x.mu = cn(c)[C_MU];
+    x.mu_hat = cn(c)[C_MUHAT];
+    x.factor = cn(c)[C_FACTOR];
     return x;
   }
   // -- blocked data --
@@ -215,7 +216,7 @@ __device__ void brows_times(const BWorld<NT, HT, NB>& w, const double* x, int sl
 #pragma unroll
       for (int b = 0; b < NB; ++b) s += __ldg(jr + side * NB + b) * xt[b];
     }
-    w.Cn(slot + k)[c] = s;
+    w.cn(c)[slot + k] = s;
   }
 }
 
@@ -223,7 +224,7 @@ __device__ void brows_times(const BWorld<NT, HT, NB>& w, const double* x, int sl
 // gradient and the scaled norms of the convergence test (the dense kernel's
 // evaluate, sim/contact_solve.py:4080-4136, without PD / limit terms).
 template <int NT, typename HT, int NB>
-__device__ void bevaluate(const BWorld<NT, HT, NB>& w, double out4[4]) {
+__device__ void bevaluate(const BWorld<NT, HT, NB>& w, double out4[4], double* mom) {
   const int tid = threadIdx.x;
   brows_times<NT, HT, NB>(w, w.V(V_V), C_VC);
   for (int i = tid; i < w.n; i += NT) w.V(V_TMP0)[i] = w.V(V_V)[i] - w.V(V_VSTAR)[i];
@@ -231,14 +232,14 @@ __device__ void bevaluate(const BWorld<NT, HT, NB>& w, double out4[4]) {
   double csum = 0.0;
   for (int c = tid; c < w.count; c += NT) {
     double g[3], cost;
-    project_contact(w.cc(c), w.Cn(C_VC + 0)[c], w.Cn(C_VC + 1)[c], w.Cn(C_VC + 2)[c], g, &cost, nullptr);
-    w.Cn(C_GAMMA + 0)[c] = g[0];
-    w.Cn(C_GAMMA + 1)[c] = g[1];
-    w.Cn(C_GAMMA + 2)[c] = g[2];
+    project_contact(w.cc(c), w.cn(c)[C_VC + 0], w.cn(c)[C_VC + 1], w.cn(c)[C_VC + 2], g, &cost, nullptr);
+    w.cn(c)[C_GAMMA + 0] = g[0];
+    w.cn(c)[C_GAMMA + 1] = g[1];
+    w.cn(c)[C_GAMMA + 2] = g[2];
     csum += cost;
   }
   __syncthreads();
-  double model_cost = 0.0, g2 = 0.0, p2 = 0.0, j2 = 0.0;
+  double model_cost = 0.0, m0 = 0.0, g2 = 0.0, p2 = 0.0, j2 = 0.0;
   for (int i = tid; i < w.n; i += NT) {
     const int t = i / NB, a = i - t * NB;
     const double* Ar = w.A + ((size_t)t * NB + a) * NB;
@@ -268,17 +269,18 @@ __device__ void bevaluate(const BWorld<NT, HT, NB>& w, double out4[4]) {
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u)
-          imp += jv[u][0] * w.Cn(C_GAMMA + 0)[cc[u]] + jv[u][1] * w.Cn(C_GAMMA + 1)[cc[u]] +
-                 jv[u][2] * w.Cn(C_GAMMA + 2)[cc[u]];
+          imp += jv[u][0] * w.cn(cc[u])[C_GAMMA + 0] + jv[u][1] * w.cn(cc[u])[C_GAMMA + 1] +
+                 jv[u][2] * w.cn(cc[u])[C_GAMMA + 2];
       }
       for (; q < q1; ++q) {
         const int c = w.list[q] >> 1, side = w.list[q] & 1;
         const double* j0 = w.jrow(c, 0) + side * NB + a;
-        imp += __ldg(j0) * w.Cn(C_GAMMA + 0)[c] + __ldg(j0 + 2 * NB) * w.Cn(C_GAMMA + 1)[c] +
-               __ldg(j0 + 4 * NB) * w.Cn(C_GAMMA + 2)[c];
+        imp += __ldg(j0) * w.cn(c)[C_GAMMA + 0] + __ldg(j0 + 2 * NB) * w.cn(c)[C_GAMMA + 1] +
+               __ldg(j0 + 4 * NB) * w.cn(c)[C_GAMMA + 2];
       }
     }
     double mc = 0.5 * w.V(V_TMP0)[i] * a_res;
+    m0 += mc;
     if (w.terms) {  // drive and limit terms (as the dense solve's evaluate)
       const double vi = vt[a], dt = w.dt;
       const int fl = w.flags[i];
@@ -325,21 +327,23 @@ __device__ void bevaluate(const BWorld<NT, HT, NB>& w, double out4[4]) {
       j2 += js * js;
     }
   }
-  double r[4] = {csum + model_cost, g2, p2, j2};
-  block_sum<NT, 4>(r, w.red);
+  double r[5] = {csum + model_cost, g2, p2, j2, m0};
+  block_sum<NT, 5>(r, w.red);
   out4[0] = r[0];
   out4[1] = r[1];
   out4[2] = r[2];
   out4[3] = r[3];
+  *mom = r[4];
 }
 
 // Line coefficients (sim/contact_solve.py:2234-2263, 1657-1692): dvc = J dv,
-// dp = A dv and {dell0, dell_a0, d2ell_a, mom0}.
+// dp = A dv and this thread's shares of {dell0, dell_a0, d2ell_a}, which the
+// line search sums with its first trials; the barrier publishes dvc.
 template <int NT, typename HT, int NB>
-__device__ void line_coefficients(const BWorld<NT, HT, NB>& w, double c4[4]) {
+__device__ void line_coefficients(const BWorld<NT, HT, NB>& w, double (&cp)[3]) {
   const int tid = threadIdx.x;
   brows_times<NT, HT, NB>(w, w.V(V_DV), C_DVC);
-  double d0 = 0.0, da0 = 0.0, d2 = 0.0, m0 = 0.0;
+  cp[0] = cp[1] = cp[2] = 0.0;
   const double* v = w.V(V_V);
   const double* vs = w.V(V_VSTAR);
   const double* dv = w.V(V_DV);
@@ -350,18 +354,11 @@ __device__ void line_coefficients(const BWorld<NT, HT, NB>& w, double c4[4]) {
 #pragma unroll
     for (int b = 0; b < NB; ++b) acc += __ldg(Ar + b) * dv[t * NB + b];
     w.V(V_DP)[i] = acc;
-    const double ri = v[i] - vs[i];
-    d0 += w.V(V_GRAD)[i] * dv[i];
-    da0 += acc * ri;
-    d2 += dv[i] * acc;
-    m0 += 0.5 * ri * w.V(V_ARES)[i];
+    cp[0] += w.V(V_GRAD)[i] * dv[i];
+    cp[1] += acc * (v[i] - vs[i]);
+    cp[2] += dv[i] * acc;
   }
-  double r[4] = {d0, da0, d2, m0};
-  block_sum<NT, 4>(r, w.red);  // its barriers also publish dvc / dp
-  c4[0] = r[0];
-  c4[1] = r[1];
-  c4[2] = r[2];
-  c4[3] = r[3];
+  __syncthreads();
 }
 
 // Element idx (row k: k * 2 NB + side * NB + column) of contact c's J row
@@ -413,7 +410,7 @@ __device__ void bassemble(const BWorld<NT, HT, NB>& w, double diag_shift) {
   if (tid == 0) w.iw[BI_MISC + 2] = 0;  // bad-pivot flag of the factorization that follows
   for (int c = tid; c < w.count; c += NT) {
     double g[3], cost, G[9];
-    project_contact(w.cc(c), w.Cn(C_VC + 0)[c], w.Cn(C_VC + 1)[c], w.Cn(C_VC + 2)[c], g, &cost, G);
+    project_contact(w.cc(c), w.cn(c)[C_VC + 0], w.cn(c)[C_VC + 1], w.cn(c)[C_VC + 2], g, &cost, G);
 #pragma unroll
     for (int k = 0; k < 9; ++k) w.G[9 * c + k] = HT(G[k]);
   }
@@ -795,9 +792,9 @@ __device__ bool bsymbolic(const BWorld<NT, HT, NB>& w, int cap) {
 template <int NT, typename HT, int NB, int LSV>
 __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double red[8 * (NT / 32)];
+  __shared__ double red[2 * kRedBatch * (NT / 32)];
   __shared__ int s_next;
-  __shared__ int s_tstart[kBMaxTrees], s_tcount[kBMaxTrees];
+  __shared__ int16_t s_tstart[kBMaxTrees], s_tcount[kBMaxTrees];  // world DOFs: at most 64 x 12
   __shared__ int s_bad_layout;
   const int tid = threadIdx.x;
   const int T = P.p.trees_per_env, C = P.p.max_contacts;
@@ -822,8 +819,8 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
       st = 0;
       cnt = 0;
     }
-    s_tstart[t] = st;
-    s_tcount[t] = cnt;
+    s_tstart[t] = (int16_t)st;
+    s_tcount[t] = (int16_t)cnt;
   }
   __syncthreads();
   auto gidx = [&](int i) {
@@ -885,14 +882,14 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
       const double tau = P.p.tau_d ? P.p.tau_d[ci] : P.o.contact_tau_d;
       const ContactConst cc = make_contact_const(P.p.phi0[ci], P.p.w_eff[ci], P.p.mu[ci], P.p.stiffness[ci], tau,
                                                  P.o.contact_beta, P.o.contact_sigma, dt);
-      w.Cn(C_RT)[c] = cc.rt;
-      w.Cn(C_RN)[c] = cc.rn;
-      w.Cn(C_RTINV)[c] = cc.rt_inv;
-      w.Cn(C_RNINV)[c] = cc.rn_inv;
-      w.Cn(C_VHAT)[c] = cc.vhat_n;
-      w.Cn(C_MU)[c] = cc.mu;
-      w.Cn(C_MUHAT)[c] = cc.mu_hat;
-      w.Cn(C_FACTOR)[c] = cc.factor;
+      w.cn(c)[C_RT] = cc.rt;
+      w.cn(c)[C_RN] = cc.rn;
+      w.cn(c)[C_RTINV] = cc.rt_inv;
+      w.cn(c)[C_RNINV] = cc.rn_inv;
+      w.cn(c)[C_VHAT] = cc.vhat_n;
+      w.cn(c)[C_MU] = cc.mu;
+      w.cn(c)[C_MUHAT] = cc.mu_hat;
+      w.cn(c)[C_FACTOR] = cc.factor;
       int t0 = P.p.contact_tree[2 * ci], t1 = P.p.contact_tree[2 * ci + 1];
       if (t0 < 0 || t0 >= T) t0 = -1;
       if (t1 < 0 || t1 >= T || t1 == t0) t1 = -1;
@@ -927,7 +924,7 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
     }
     for (int k = tid; k < count * 6 * NB; k += NT) bad = bad || !isfinite(__ldg(w.J + k));
     for (int c = tid; c < count; c += NT)  // the contact constants formed above
-      for (int q = C_RT; q < C_VC; ++q) bad = bad || !isfinite(w.Cn(q)[c]);
+      for (int q = C_RT; q < C_VC; ++q) bad = bad || !isfinite(w.cn(c)[q]);
     bad = __syncthreads_or(bad) != 0;
     w.dt = dt;
     // drive and limit terms of the world's own DOFs (sim/contact_solve.py:
@@ -1070,11 +1067,13 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
       // cost is below the plain start's; its evaluation then seeds
       // iteration 0.
       bool have_e4 = false;
+      double mom = 0.0;  // 1/2 (v - v*) A (v - v*) of the last evaluation
       double e4_seed[4] = {0.0, 0.0, 0.0, 0.0};
       if (P.p.gamma0) {
-        double e4p[4];
-        bevaluate<NT, HT, NB>(w, e4p);
+        double e4p[4], m_unused;
+        bevaluate<NT, HT, NB>(w, e4p, &m_unused);
         for (int i = tid; i < n; i += NT) w.V(V_SAVE)[i] = w.V(V_V)[i];
+        __syncthreads();  // (a tree's thread writes what other threads save)
         for (int t = tid; t < T; t += NT) {
           const int q0 = w.iw[BI_CSTART + t], q1 = w.iw[BI_CSTART + t + 1];
           if (q1 == q0) continue;  // no contact: v* already
@@ -1125,11 +1124,12 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
           for (int a = 0; a < NB; ++a) w.V(V_V)[t * NB + a] = w.V(V_VSTAR)[t * NB + a] + r[a];
         }
         __syncthreads();
-        double e4c[4];
-        bevaluate<NT, HT, NB>(w, e4c);
+        double e4c[4], m_c;
+        bevaluate<NT, HT, NB>(w, e4c, &m_c);
         if (e4c[0] < e4p[0]) {
           accepted = 1;
           have_e4 = true;
+          mom = m_c;
           for (int q = 0; q < 4; ++q) e4_seed[q] = e4c[q];
         } else {
           for (int i = tid; i < n; i += NT) w.V(V_V)[i] = w.V(V_SAVE)[i];
@@ -1143,7 +1143,7 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
           for (int q = 0; q < 4; ++q) e4[q] = e4_seed[q];
           have_e4 = false;
         } else {
-          bevaluate<NT, HT, NB>(w, e4);
+          bevaluate<NT, HT, NB>(w, e4, &mom);
         }
         evaluated = true;
         cost = e4[0];
@@ -1167,15 +1167,15 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
         bassemble<NT, HT, NB>(w, P.o.diag_shift);
         bfactor<NT, HT, NB>(w);
         bsolve<NT, HT, NB>(w);
-        double c4[4];
-        line_coefficients<NT, HT, NB>(w, c4);
+        double cp[3];
+        line_coefficients<NT, HT, NB>(w, cp);
         LsResult r;
         if constexpr (LSV == SAPB_LS_ARMIJO_DECAY)
-          r = ls_armijo<NT, 1>(w, P, dt, cost, c4);
+          r = ls_armijo<NT, 1>(w, P, dt, cost, cp, mom);
         else if constexpr (LSV == SAPB_LS_EXACT_ROOT)
-          r = ls_exact<NT>(w, P, dt, cost, c4);
+          r = ls_exact<NT>(w, P, dt, cost, cp, mom);
         else
-          r = ls_monotone<NT, 1>(w, P, dt, cost, c4);
+          r = ls_monotone<NT, 1>(w, P, dt, cost, cp, mom);
         alpha = r.alpha;
         status = r.status;
         constexpr bool mono = LSV == SAPB_LS_MONOTONE_DECAY;
@@ -1198,15 +1198,15 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
       const size_t ci = (size_t)e * C + c;
       const bool live = evaluated && c < count;
       if (P.out.contact_gamma) {
-        P.out.contact_gamma[ci * 3 + 0] = live ? w.Cn(C_GAMMA + 0)[c] : 0.0;
-        P.out.contact_gamma[ci * 3 + 1] = live ? w.Cn(C_GAMMA + 1)[c] : 0.0;
-        P.out.contact_gamma[ci * 3 + 2] = live ? w.Cn(C_GAMMA + 2)[c] : 0.0;
+        P.out.contact_gamma[ci * 3 + 0] = live ? w.cn(c)[C_GAMMA + 0] : 0.0;
+        P.out.contact_gamma[ci * 3 + 1] = live ? w.cn(c)[C_GAMMA + 1] : 0.0;
+        P.out.contact_gamma[ci * 3 + 2] = live ? w.cn(c)[C_GAMMA + 2] : 0.0;
       }
       if (P.out.contact_mode) {
         int mode = SAPB_CONTACT_MODE_NONE;
         if (live) {
           double g[3], cst;
-          mode = project_contact(w.cc(c), w.Cn(C_VC + 0)[c], w.Cn(C_VC + 1)[c], w.Cn(C_VC + 2)[c], g, &cst, nullptr);
+          mode = project_contact(w.cc(c), w.cn(c)[C_VC + 0], w.cn(c)[C_VC + 1], w.cn(c)[C_VC + 2], g, &cst, nullptr);
         }
         P.out.contact_mode[ci] = mode;
       }

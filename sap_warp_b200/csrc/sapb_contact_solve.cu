@@ -6,12 +6,14 @@
 namespace sapb {
 
 size_t contact_solve_smem_bytes(int n, int C, int hessian_precision, int threads) {
-  return make_layout(n, C, hessian_precision == SAPB_FP32 ? 4 : 8, (threads > 0 ? threads : 128) / 32).total;
+  return make_layout(n, C, hessian_precision == SAPB_FP32 ? 4 : 8, threads > 0 ? threads : 128).total;
 }
 
 // Resident CTAs per SM of the kernel a problem of this shape launches: the
 // same dispatch with num_envs = 0, which stops at the occupancy query.
 static cudaError_t solve_dispatch(const SolveParams& P, bool fp32, cudaStream_t stream, int* blocks_out);
+
+constexpr int kSolveCounters = 5;  // within the 256 bytes of workspace
 
 int32_t contact_solve_occupancy(int n, int C, int hessian_precision, int variant, int threads) {
   if (n < 1 || C < 0) return SAPB_ERR_INVALID_ARGUMENT;
@@ -50,15 +52,8 @@ int ldlt_block_widths(int n, int32_t* out, int capacity) {
   }
 }
 
-static cudaError_t solve_dispatch(const SolveParams& P, bool fp32, cudaStream_t stream, int* blocks_out) {
-  // Kernels specialised on the DOF count of the common trees (humanoid 35,
-  // quadruped 18, arm + box 13, single free body 6); a generic one otherwise
-  // and for per-world DOF counts; the generic one with eight warps per world
-  // on request.
-  if (P.o.threads_per_cta == 256)
-    return fp32 ? launch_solve_wide<true>(P, stream, blocks_out) : launch_solve_wide<false>(P, stream, blocks_out);
-  if (P.p.dof_count) return launch_solve_ns<0>(P, fp32, stream, blocks_out);
-  switch (P.p.dof_per_env) {
+static cudaError_t solve_sized(const SolveParams& P, int n, bool fp32, cudaStream_t stream, int* blocks_out) {
+  switch (n) {
 #define SAPB_DISPATCH_N(NV) \
   case NV:                  \
     return launch_solve_ns<NV>(P, fp32, stream, blocks_out);
@@ -70,6 +65,36 @@ static cudaError_t solve_dispatch(const SolveParams& P, bool fp32, cudaStream_t 
     default:
       return launch_solve_ns<0>(P, fp32, stream, blocks_out);
   }
+}
+
+static cudaError_t solve_dispatch(const SolveParams& P, bool fp32, cudaStream_t stream, int* blocks_out) {
+  // Kernels specialised on the DOF count of the common trees (humanoid 35,
+  // quadruped 18, arm + box 13, single free body 6); a generic one otherwise;
+  // the generic one with eight warps per world on request.
+  if (P.o.threads_per_cta == 256)
+    return fp32 ? launch_solve_wide<true>(P, stream, blocks_out) : launch_solve_wide<false>(P, stream, blocks_out);
+  if (!P.p.dof_count) return solve_sized(P, P.p.dof_per_env, fp32, stream, blocks_out);
+  // Per-world DOF counts: one launch per size class, each kernel taking the
+  // worlds of its class from the order, the largest first.  The kernel that
+  // holds every class's code spills 2 KB of registers and overruns the
+  // instruction cache (6000 worlds of 13, 18 and 35 DOFs, FP32: 1389 us, the
+  // classes' launches 1047 us), but runs small batches' classes side by side,
+  // where a launch's time is its longest world's (192 worlds: 293 us and 377
+  // us; 1500: 506 us and 545 us).
+  int dev = 0, sms = 0;
+  cudaError_t err = cudaGetDevice(&dev);
+  if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (err != cudaSuccess) return err;
+  if (P.p.num_envs <= 16 * sms) return launch_solve_ns<kMixed>(P, fp32, stream, blocks_out);
+  SolveParams Q = P;
+  Q.own_class_only = 1;
+  for (int n : {35, 18, 13, 6, 0}) {
+    if (n > P.p.dof_per_env) continue;
+    err = solve_sized(Q, n, fp32, stream, nullptr);
+    if (err != cudaSuccess) return err;
+    ++Q.queue;
+  }
+  return cudaSuccess;
 }
 
 int32_t contact_solve_launch(const sapb_contact_problem* p, const sapb_solve_options* o, const sapb_solve_outputs* out,
@@ -94,7 +119,9 @@ int32_t contact_solve_launch(const sapb_contact_problem* p, const sapb_solve_opt
                    (size_t)kMaxSmemPerBlock);
     return SAPB_ERR_UNSUPPORTED;
   }
-  const cudaError_t err = solve_dispatch(P, fp32, stream, nullptr);
+  // the work counters, one for each size class
+  cudaError_t err = cudaMemsetAsync(P.queue, 0, kSolveCounters * sizeof(int32_t), stream);
+  if (err == cudaSuccess) err = solve_dispatch(P, fp32, stream, nullptr);
   if (err != cudaSuccess) {
     set_last_error("contact solve launch: %s", cudaGetErrorString(err));
     return SAPB_ERR_CUDA;

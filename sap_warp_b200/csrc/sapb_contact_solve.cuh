@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstring>
 #include <type_traits>
+#include <utility>
 
 #include "sapb_device.cuh"
 #include "sapb_internal.h"
@@ -37,66 +38,80 @@ struct SolveParams {
   sapb_solve_outputs out;
   int32_t use_guess_flag_ptr_valid;
   int32_t* queue;      // work counter (zeroed before launch)
+  // batches of per-world DOF counts in one launch per size class: this kernel
+  // takes only its class (the runtime-size kernel the worlds of none)
+  int32_t own_class_only;
 };
 
-__host__ __device__ inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+// DOF counts with a specialised kernel: humanoid, quadruped, arm + box, one
+// free body.
+__host__ __device__ constexpr bool specialised_dofs(int n) { return n == 35 || n == 18 || n == 13 || n == 6; }
 
-// Shared-memory layout of one world.  ldJ: room for the 4-wide Hessian tiles
-// and odd, so thread-per-row reads of J are free of bank conflicts.  ldH odd
-// for conflict-free column reads in the factorization.
-struct Layout {
-  int n, C, ldJ, ldH, nb, nw;
-  size_t off_J, off_scr, off_H, off_G, off_vec, off_con, off_flags, off_tri, total;
-  static constexpr int kVecs = 23;
-  static constexpr int kConPer = 17;
-  static constexpr int kMinWarps = 4;  // partial-sum scratch of at least four warps
+// Shared-memory layout of one world: the factorization's triangle list (of
+// the kernel's largest world), the arrays sized by the world's DOFs alone --
+// at compile-time offsets from one base in the specialised kernels, so that
+// their addresses cost neither registers nor instructions -- then those sized
+// by the contact slots.  ldJ and ldH odd: thread-per-row reads of J and column
+// reads of H in the factorization are free of bank conflicts.
+constexpr int kVecs = V_END;
+
+__host__ __device__ constexpr size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
+
+struct FixedLayout {
+  int ps;  // one row of partial sums: up to eight chunks of n
+  size_t off_scr, off_H, off_vec, off_flags, total;
 };
-
-// warps: of the CTA (the partial-sum scratch holds one row per warp)
-__host__ __device__ inline Layout make_layout(int n, int C, int hsize, int warps = 4) {
-  Layout L;
-  L.n = n;
-  L.C = C;
-  L.nw = warps > Layout::kMinWarps ? warps : Layout::kMinWarps;
-  L.ldJ = (n + 3) / 4 * 4 + 1;
-  L.ldH = (n % 2 == 0) ? n + 1 : n;
-  L.nb = (n + 3) / 4;
+// threads: of the CTA (the DOF products' partial sums hold one row per chunk)
+__host__ __device__ constexpr FixedLayout fixed_layout(int n, int hsize, int threads) {
+  FixedLayout L{};
+  const size_t ld = n | 1;
+  L.ps = n <= 8 || 8 * n > threads ? threads : 8 * n;
   size_t o = 0;
-  L.off_J = o;
-  o = align_up(o + sizeof(double) * (size_t)3 * C * L.ldJ, 16);
-  L.off_scr = o;  // the partial sums of the DOF products, or two staged impulse sets
-  {
-    const size_t part = sizeof(double) * 3 * (size_t)L.nw * 64;
-    const size_t gam = sizeof(double) * 6 * (size_t)(C > 0 ? C : 1);
-    o = align_up(o + (part > gam ? part : gam), 16);
-  }
-  L.off_H = o;
-  o = align_up(o + (size_t)hsize * n * L.ldH, 16);
-  L.off_G = o;
-  o = align_up(o + (size_t)hsize * 9 * (size_t)(C > 0 ? C : 1), 16);
+  L.off_scr = o;  // in turn: two rows of partial sums, the factorization's scaled panel
+  const size_t sums = sizeof(double) * 2 * (size_t)L.ps, pan = (size_t)hsize * 8 * (n + 1);
+  o = align_up(o + (sums > pan ? sums : pan), 16);
+  L.off_H = o;  // n rows, then the right-hand side
+  o = align_up(o + (size_t)hsize * (n + 1) * ld, 16);
   L.off_vec = o;
-  o = align_up(o + sizeof(double) * (size_t)Layout::kVecs * L.ldJ, 16);
-  L.off_con = o;
-  o = align_up(o + sizeof(double) * (size_t)Layout::kConPer * (C > 0 ? C : 1), 16);
+  o = align_up(o + sizeof(double) * (size_t)kVecs * ld, 16);
   L.off_flags = o;
-  o = align_up(o + sizeof(int) * (size_t)L.ldJ, 16);
-  L.off_tri = o;  // (i << 8 | j) of the lower triangle below row 0, columns descending
-  o = align_up(o + sizeof(uint16_t) * (size_t)(n * (n - 1) / 2 + 1), 16);
+  o = align_up(o + sizeof(int) * ld, 16);
   L.total = o;
   return L;
 }
 
-static_assert(V_END <= Layout::kVecs, "vector slots");
-static_assert(C_END <= Layout::kConPer, "contact slots");
+struct Layout {
+  int n, C;
+  size_t off_fixed, off_con, off_G, off_J, total;
+};
+__host__ __device__ inline Layout make_layout(int n, int C, int hsize, int threads = 128) {
+  Layout L;
+  L.n = n;
+  L.C = C;
+  const size_t Cc = C > 0 ? C : 1;
+  size_t o = align_up(sizeof(uint16_t) * (size_t)triangle_list_size(n, 1), 16);  // the list, at 0
+  L.off_fixed = o;
+  // (a mixed batch's six-DOF worlds use their own fixed layout in this place)
+  const size_t own = fixed_layout(n, hsize, threads).total, six = n > 6 ? fixed_layout(6, hsize, threads).total : 0;
+  o += own > six ? own : six;
+  L.off_con = o;
+  o += sizeof(double) * C_END * Cc;
+  L.off_G = o;  // (before the first evaluation: two staged impulse sets)
+  o += sizeof(double) * 9 * Cc;
+  L.off_J = o;
+  L.total = align_up(o + sizeof(double) * (size_t)3 * C * (n | 1), 16);
+  return L;
+}
 
 template <int NT, typename HT, int NS>
 struct World {
-  Layout L;
+  static constexpr int kCoefWarps = 1;  // warp 0 holds the line coefficients' shares
+  int n_list, ps;   // DOFs of the triangle list; doubles in a row of partial sums
   const double* A;  // global, this world's [n][n]
   double* J;
-  HT* GJ;           // scratch: the partial sums of the DOF products, or staged impulse sets
+  double* scr;      // scratch: partial sums or the scaled panel
   HT* H;
-  HT* G;            // [C][9], in the Hessian's type
+  double* G;        // [C][9]
   double* vec;
   double* con;
   int* flags;
@@ -106,172 +121,257 @@ struct World {
   int n, count;
   // DOF count and leading dimensions: compile-time constants when NS > 0.
   __device__ __forceinline__ int dofs() const { return NS > 0 ? NS : n; }
-  __device__ __forceinline__ int ldJ() const { return NS > 0 ? (NS + 3) / 4 * 4 + 1 : L.ldJ; }
-  __device__ __forceinline__ int ldH() const { return NS > 0 ? ((NS % 2 == 0) ? NS + 1 : NS) : L.ldH; }
-  __device__ __forceinline__ int nb() const { return NS > 0 ? (NS + 3) / 4 : (n + 3) / 4; }
+  __device__ __forceinline__ int ldJ() const { return NS > 0 ? NS | 1 : n | 1; }
+  __device__ __forceinline__ int ldH() const { return NS > 0 ? NS | 1 : n | 1; }
   // shift of the kernel's triangle list (built for L.n DOFs) to this world's n
-  __device__ __forceinline__ int tri_shift() const { return L.n - dofs(); }
-  __device__ double* V(int k) const { return vec + (size_t)k * ldJ(); }
-  __device__ double* Cn(int k) const { return con + (size_t)k * L.C; }
-  __device__ double* part(int which, int warp) const {
-    return reinterpret_cast<double*>(GJ) + ((size_t)which * L.nw + warp) * 64;
-  }
+  __device__ __forceinline__ int tri_shift() const { return n_list - dofs(); }
+  __device__ __forceinline__ double* V(int k) const { return vec + k * ldJ(); }
+  __device__ __forceinline__ double* cn(int c) const { return con + c * (int)C_END; }
+  __device__ double* part(int which) const { return scr + which * ps; }
   __device__ ContactConst cc(int c) const {
     ContactConst x;
-    x.rt = Cn(C_RT)[c];
-    x.rn = Cn(C_RN)[c];
-    x.rt_inv = Cn(C_RTINV)[c];
-    x.rn_inv = Cn(C_RNINV)[c];
-    x.vhat_n = Cn(C_VHAT)[c];
-    x.mu = Cn(C_MU)[c];
-    x.mu_hat = Cn(C_MUHAT)[c];
-    x.factor = Cn(C_FACTOR)[c];
+    x.rt = cn(c)[C_RT];
+    x.rn = cn(c)[C_RN];
+    x.rt_inv = cn(c)[C_RTINV];
+    x.rn_inv = cn(c)[C_RNINV];
+    x.vhat_n = cn(c)[C_VHAT];
+    x.mu = cn(c)[C_MU];
+    x.mu_hat = cn(c)[C_MUHAT];
+    x.factor = cn(c)[C_FACTOR];
     return x;
   }
 };
 
-// vc-type products: rows r < 3*count of J times x (length n, shared) into the
-// contact slots `slot..slot+2`.  One thread per row.
+// The DOF products run on NT threads as (DOF i, chunk ch): thread t holds DOF
+// t % n of chunk t / n, so consecutive threads read consecutive addresses and
+// up to NT / n chunks of the summed index run side by side (35 DOFs: three
+// chunks on 105 threads).
 template <int NT, typename HT, int NS>
-__device__ void contact_rows_times(const World<NT, HT, NS>& w, const double* x, int slot) {
-  const int rows = 3 * w.count;
-  for (int r = threadIdx.x; r < rows; r += NT) {
-    const double* row = w.J + (size_t)r * w.ldJ();
+struct DofChunks {
+  int i, ch, count;  // this thread's DOF and chunk (ch >= count: none), chunks
+  __device__ __forceinline__ explicit DofChunks(const World<NT, HT, NS>& w) {
+    const int n = w.dofs();
+    count = NT / n < 8 ? NT / n : 8;
+    ch = (int)threadIdx.x / n;
+    i = (int)threadIdx.x - ch * n;
+  }
+  __device__ __forceinline__ bool active() const { return ch < count; }
+};
+
+// vc-type products: rows r < 3*count of J times x (length n, shared) into the
+// contact slots `slot..slot+2`.  Two neighbouring threads per row, each half
+// of the columns (20 contacts' rows are then one pass of 120 threads).
+template <int NT, typename HT, int NS>
+__device__ __forceinline__ void contact_rows_times(const World<NT, HT, NS>& w, const double* x, int slot) {
+  const int n = w.dofs(), h = (n + 1) / 2;
+  const int half = threadIdx.x & 1, j0 = half ? h : 0;
+  const int items = 2 * 3 * w.count;
+#pragma unroll 1
+  for (int t0 = 0; t0 < items; t0 += NT) {
+    const int t = t0 + (int)threadIdx.x, r = t >> 1;
     double s0 = 0.0, s1 = 0.0;
-    int j = 0;
-    for (; j + 1 < w.dofs(); j += 2) {
-      s0 += row[j] * x[j];
-      s1 += row[j + 1] * x[j + 1];
+    if (t < items) {
+      const double* row = w.J + r * w.ldJ() + j0;
+      const double* xh = x + j0;
+      int j = 0;
+#pragma unroll 6
+      for (; j + 1 < h - 1; j += 2) {
+        s0 += row[j] * xh[j];
+        s1 += row[j + 1] * xh[j + 1];
+      }
+      for (; j < h - (n & half); ++j) s0 += row[j] * xh[j];  // (odd n: the second half is one shorter)
+      s0 += s1;
     }
-    if (j < w.dofs()) s0 += row[j] * x[j];
-    const int c = r / 3, k = r - 3 * c;
-    w.Cn(slot + k)[c] = s0 + s1;
+    s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+    if (t < items && half == 0) {
+      const int c = r / 3, k = r - 3 * c;
+      w.cn(c)[slot + k] = s0;
+    }
   }
 }
 
-// Partial sums of the per-DOF products over a warp's share of the columns of
-// A and of the contacts: part(0)[i] = sum_j A[j][i] x[j], part(1)[i] =
-// sum_j A[j][i] y[j], part(2)[i] = sum_c J_c[:, i] . gamma_c.  Lanes own DOFs
-// i = lane and lane + 32, so a warp reads consecutive addresses.
+// part(0) <- chunk sums of A x (x = V_DV), or of A (v - v*) with `residual`;
+// part(1) <- chunk sums of A v* with `vstar_too`.
 template <int NT, typename HT, int NS>
-__device__ void dof_partials(const World<NT, HT, NS>& w, const double* x, const double* y, bool with_gamma) {
-  constexpr int NW = NT / 32;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__device__ __forceinline__ void a_partials(const World<NT, HT, NS>& w, bool residual, bool vstar_too) {
+  const DofChunks<NT, HT, NS> k(w);
+  if (!k.active()) return;
   const int n = w.dofs();
-  const int jchunk = (n + NW - 1) / NW;
-  const int j0 = warp * jchunk, j1 = min(n, j0 + jchunk);
-  const int cchunk = (w.count + NW - 1) / NW;
-  const int c0 = warp * cchunk, c1 = min(w.count, c0 + cchunk);
-#pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int i = lane + 32 * h;
-    if (i >= n) continue;
-    double a = 0.0, b = 0.0, g = 0.0;
-    for (int j = j0; j < j1; ++j) {
-      const double aij = __ldg(w.A + (size_t)j * n + i);
-      a += aij * x[j];
-      if (y) b += aij * y[j];
-    }
-    if (with_gamma) {
-      const int ld = w.ldJ();
-      for (int c = c0; c < c1; ++c) {
-        const double* Jc = w.J + (size_t)(3 * c) * ld + i;
-        g += Jc[0] * w.Cn(C_GAMMA + 0)[c] + Jc[ld] * w.Cn(C_GAMMA + 1)[c] + Jc[2 * ld] * w.Cn(C_GAMMA + 2)[c];
-      }
-    }
-    w.part(0, warp)[i] = a;
-    w.part(1, warp)[i] = b;
-    w.part(2, warp)[i] = g;
+  const int per = (n + k.count - 1) / k.count;
+  const int j0 = k.ch * per, j1 = min(n, j0 + per);
+  const double *x = w.V(residual ? V_V : V_DV), *vs = w.V(V_VSTAR);
+  double a = 0.0, b = 0.0;
+#pragma unroll 4
+  for (int j = j0; j < j1; ++j) {
+    const double aij = __ldg(w.A + (size_t)j * n + k.i);
+    a += aij * (residual ? x[j] - vs[j] : x[j]);
+    if (vstar_too) b += aij * vs[j];
   }
+  w.part(0)[k.ch * n + k.i] = a;
+  if (vstar_too) w.part(1)[k.ch * n + k.i] = b;
 }
 
 template <int NT, typename HT, int NS>
 __device__ __forceinline__ double sum_partials(const World<NT, HT, NS>& w, int which, int i) {
-  constexpr int NW = NT / 32;
-  double s = 0.0;
-#pragma unroll
-  for (int k = 0; k < NW; ++k) s += w.part(which, k)[i];
+  const int n = w.dofs(), nch = NT / n < 8 ? NT / n : 8;
+  const double* p = w.part(which) + i;
+  double s = p[0];
+  for (int k = 1; k < nch; ++k) s += p[k * n];
   return s;
 }
 
-// Objective at the current v (shared V_V): contact gamma and cost, A(v-v*),
-// J^T gamma, PD and limit terms, gradient.  Returns {cost, |g|^2, |p|^2, |jc|^2}
-// (scaled, over participating DOFs) to every thread.  Restates
-// _solver_update_active sim/contact_solve.py:4080-4136.
+enum EvalStart { kEvalFull = 0, kEvalStep = 1, kEvalSame = 2 };
+
+// Objective at the current v: contact impulses, costs and derivatives G,
+// a_res = A(v - v*), J^T gamma, PD and limit terms, gradient (and its negative
+// as the factorization's right-hand-side row).  Returns {cost, |g|^2, |p|^2,
+// |jc|^2} (scaled, over participating DOFs) and the momentum cost
+// 1/2 (v - v*) a_res to every thread.  Restates _solver_update_active
+// sim/contact_solve.py:4080-4136.
+//
+// kEvalFull forms vc = J v and a_res from V_V; kEvalStep moves v, vc and
+// a_res by alpha times dv, J dv and A dv of the line search (all linear in v:
+// a Newton step then reads neither A nor J here but for J^T gamma); kEvalSame
+// leaves them.  The first two warps hold the DOFs; of the others every second
+// one projects the contacts for impulses and costs and the rest for the
+// derivatives, side by side (the projection is a long dependent chain of few
+// threads).
 template <int NT, typename HT, int NS>
-__device__ void evaluate(const World<NT, HT, NS>& w, const SolveParams& P, double dt, double out4[4]) {
-  const int tid = threadIdx.x;
-  contact_rows_times<NT, HT, NS>(w, w.V(V_V), C_VC);
-  for (int i = tid; i < w.dofs(); i += NT) w.V(V_TMP0)[i] = w.V(V_V)[i] - w.V(V_VSTAR)[i];
+__device__ __forceinline__ void evaluate(const World<NT, HT, NS>& w, const SolveParams& P, double dt, int start,
+                                         bool first, double alpha, double out4[4], double* mom) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int NW = NT / 32, kStride = 32 * (NW - 2) / 2;
+  const int n = w.dofs();
+  if (start == kEvalFull) {
+    contact_rows_times<NT, HT, NS>(w, w.V(V_V), C_VC);
+    a_partials<NT, HT, NS>(w, true, first);
+    __syncthreads();
+  }
+  if (warp < 2) {
+    if (tid < n) {
+      if (start == kEvalFull) {
+        w.V(V_ARES)[tid] = sum_partials<NT, HT, NS>(w, 0, tid);
+        if (first) w.V(V_AVS)[tid] = sum_partials<NT, HT, NS>(w, 1, tid);
+      } else if (start == kEvalStep) {
+        w.V(V_V)[tid] += alpha * w.V(V_DV)[tid];
+        w.V(V_ARES)[tid] += alpha * w.V(V_DP)[tid];
+      }
+    }
+  } else {
+    const bool derivs = warp & 1;
+    double csum = 0.0;
+#pragma unroll 1
+    for (int c = 32 * ((warp - 2) >> 1) + lane; c < w.count; c += kStride) {
+      double vc[3], g[3], cost, G[9];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        vc[k] = w.cn(c)[C_VC + k];
+        if (start == kEvalStep) vc[k] += alpha * w.cn(c)[C_DVC + k];
+      }
+      if (derivs) {
+        project_contact(w.cc(c), vc[0], vc[1], vc[2], g, &cost, G);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) w.G[9 * c + k] = G[k];
+      } else {
+        project_contact(w.cc(c), vc[0], vc[1], vc[2], g, &cost, nullptr);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) w.cn(c)[C_GAMMA + k] = g[k];
+        csum += cost;
+      }
+    }
+    if (!derivs) {
+      csum = warp_sum<NT>(csum);
+      if (lane == 0) w.red[kRedCost * NW + warp] = csum;
+    }
+  }
   __syncthreads();
+  {  // J^T gamma over chunks of the contacts
+    const DofChunks<NT, HT, NS> k(w);
+    if (k.active()) {
+      const int per = (w.count + k.count - 1) / k.count;
+      const int c0 = k.ch * per, c1 = min(w.count, c0 + per);
+      const int ld = w.ldJ();
+      double g0 = 0.0, g1 = 0.0, g2 = 0.0;
+      const double* Jc = w.J + 3 * c0 * ld + k.i;
+#pragma unroll 2
+      for (int c = c0; c < c1; ++c, Jc += 3 * ld) {
+        g0 += Jc[0] * w.cn(c)[C_GAMMA + 0];
+        g1 += Jc[ld] * w.cn(c)[C_GAMMA + 1];
+        g2 += Jc[2 * ld] * w.cn(c)[C_GAMMA + 2];
+      }
+      w.part(0)[k.ch * n + k.i] = (g0 + g1) + g2;
+    }
+  }
+  __syncthreads();
+  if (warp == 0) {  // gradient and norms: two DOFs a lane
+    double mterm = 0.0, extra = 0.0, g2 = 0.0, p2 = 0.0, j2 = 0.0;
+    HT* rhs = w.H + n * w.ldH();
+#pragma unroll 1
+    for (int i = lane; i < n; i += 32) {
+      double imp = sum_partials<NT, HT, NS>(w, 0, i);
+      const double a_res = w.V(V_ARES)[i], vi = w.V(V_V)[i];
+      const double a_v = a_res + w.V(V_AVS)[i];
+      mterm += 0.5 * (vi - w.V(V_VSTAR)[i]) * a_res;
+      const int fl = w.flags[i];
+      double pdg = 0.0, hd = 0.0;
+      if (P.dof.has_pd && (fl & kFlagPd)) {
+        const double gain = w.V(V_PDGAIN)[i], lim = w.V(V_PDLIM)[i];
+        const double y = w.V(V_PDA)[i] - gain * vi;
+        pdg = dt * clamp_limit(y, lim);
+        hd += dt * gain * clamp_limit_derivative(y, lim);
+        if (gain > 0.0) extra += (dt / gain) * clamp_limit_antiderivative(y, lim);
+      }
+      double lg = 0.0;
+      if (P.dof.has_limits) {
+        if (fl & kFlagLo) {
+          const double g = w.V(V_LORINV)[i] * (w.V(V_LOVHAT)[i] - vi);
+          if (g > 0.0) {
+            lg += g;
+            hd += w.V(V_LORINV)[i];
+            extra += 0.5 * w.V(V_LOR)[i] * g * g;
+          }
+        }
+        if (fl & kFlagUp) {
+          const double g = w.V(V_UPRINV)[i] * (w.V(V_UPVHAT)[i] + vi);
+          if (g > 0.0) {
+            lg -= g;
+            hd += w.V(V_UPRINV)[i];
+            extra += 0.5 * w.V(V_UPR)[i] * g * g;
+          }
+        }
+      }
+      imp += pdg + lg;
+      const double grad = a_res - imp;
+      w.V(V_GRAD)[i] = grad;
+      w.V(V_HDIAG)[i] = hd;
+      rhs[i] = HT(-grad);
+      if (fl & kFlagPart) {
+        const double s = w.V(V_DSCALE)[i];
+        const double gs = s * grad, ps = s * a_v, js = s * imp;
+        g2 += gs * gs;
+        p2 += ps * ps;
+        j2 += js * js;
+      }
+    }
+    const double tot = warp_sum4(mterm, g2, p2, j2);
+    double* r = w.red + kRedEval * NW;
+    if ((lane & 7) == 0) r[lane >> 3] = tot;
+    if (P.dof.has_pd || P.dof.has_limits) extra = warp_sum<NT>(extra);
+    if (lane == 0) r[4] = extra;
+  } else if (start == kEvalStep) {  // the moved contact velocities (their old ones are read)
+#pragma unroll 1
+    for (int q = tid - 32; q < 3 * w.count; q += NT - 32) {
+      const int k = q / w.count, c = q - k * w.count;
+      w.cn(c)[C_VC + k] += alpha * w.cn(c)[C_DVC + k];
+    }
+  }
+  __syncthreads();
+  const double* r = w.red + kRedEval * NW;
   double csum = 0.0;
-  for (int c = tid; c < w.count; c += NT) {
-    double g[3], cost;
-    project_contact(w.cc(c), w.Cn(C_VC + 0)[c], w.Cn(C_VC + 1)[c], w.Cn(C_VC + 2)[c], g, &cost, nullptr);
-    w.Cn(C_GAMMA + 0)[c] = g[0];
-    w.Cn(C_GAMMA + 1)[c] = g[1];
-    w.Cn(C_GAMMA + 2)[c] = g[2];
-    csum += cost;
-  }
-  __syncthreads();
-  dof_partials<NT, HT, NS>(w, w.V(V_TMP0), w.V(V_V), true);
-  __syncthreads();
-  double model_cost = 0.0, g2 = 0.0, p2 = 0.0, j2 = 0.0;
-  const double* v = w.V(V_V);
-  const double* vs = w.V(V_VSTAR);
-  for (int i = tid; i < w.dofs(); i += NT) {
-    const double a_res = sum_partials<NT, HT, NS>(w, 0, i);
-    const double a_v = sum_partials<NT, HT, NS>(w, 1, i);
-    double imp = sum_partials<NT, HT, NS>(w, 2, i);
-    const double vi = v[i];
-    double mc = 0.5 * (vi - vs[i]) * a_res;
-    const int fl = w.flags[i];
-    double pdg = 0.0, hd = 0.0;
-    if (P.dof.has_pd && (fl & kFlagPd)) {
-      const double gain = w.V(V_PDGAIN)[i], lim = w.V(V_PDLIM)[i];
-      const double y = w.V(V_PDA)[i] - gain * vi;
-      pdg = dt * clamp_limit(y, lim);
-      hd += dt * gain * clamp_limit_derivative(y, lim);
-      if (gain > 0.0) mc += (dt / gain) * clamp_limit_antiderivative(y, lim);
-    }
-    double lg = 0.0;
-    if (P.dof.has_limits) {
-      double lc = 0.0;
-      if (fl & kFlagLo) {
-        const double g = w.V(V_LORINV)[i] * (w.V(V_LOVHAT)[i] - vi);
-        if (g > 0.0) {
-          lg += g;
-          hd += w.V(V_LORINV)[i];
-          lc += 0.5 * w.V(V_LOR)[i] * g * g;
-        }
-      }
-      if (fl & kFlagUp) {
-        const double g = w.V(V_UPRINV)[i] * (w.V(V_UPVHAT)[i] + vi);
-        if (g > 0.0) {
-          lg -= g;
-          hd += w.V(V_UPRINV)[i];
-          lc += 0.5 * w.V(V_UPR)[i] * g * g;
-        }
-      }
-      mc += lc;
-    }
-    imp += pdg + lg;
-    const double grad = a_res - imp;
-    w.V(V_ARES)[i] = a_res;
-    w.V(V_GRAD)[i] = grad;
-    w.V(V_HDIAG)[i] = hd;
-    model_cost += mc;
-    if (fl & kFlagPart) {
-      const double s = w.V(V_DSCALE)[i];
-      const double gs = s * grad, ps = s * a_v, js = s * imp;
-      g2 += gs * gs;
-      p2 += ps * ps;
-      j2 += js * js;
-    }
-  }
-  double r[4] = {csum + model_cost, g2, p2, j2};
-  block_sum<NT, 4>(r, w.red);
-  out4[0] = r[0];
+#pragma unroll
+  for (int q = 2; q < NW; q += 2) csum += w.red[kRedCost * NW + q];
+  *mom = r[0];
+  out4[0] = (csum + r[0]) + r[4];
   out4[1] = r[1];
   out4[2] = r[2];
   out4[3] = r[3];
@@ -281,11 +381,11 @@ __device__ void evaluate(const World<NT, HT, NS>& w, const SolveParams& P, doubl
 // global memory (+ diag_add on the diagonal): flat coalesced reads, four
 // loads in flight per thread.
 template <int NT, typename HT, int NS>
-__device__ __forceinline__ void load_lower(const World<NT, HT, NS>& w, const double* M, const double* diag_add,
-                                           double shift) {
+__device__ __forceinline__ void load_lower(const World<NT, HT, NS>& w, const double* M) {
   const int tid = threadIdx.x;
   const int n = w.dofs(), ldH = w.ldH();
   const int total = n * n;
+#pragma unroll 1
   for (int k0 = tid; k0 < total; k0 += 4 * NT) {
     double val[4];
 #pragma unroll
@@ -298,133 +398,164 @@ __device__ __forceinline__ void load_lower(const World<NT, HT, NS>& w, const dou
       const int k = k0 + u * NT;
       if (k < total) {
         const int i = k / n, j = k - i * n;
-        if (j < i) w.H[(size_t)i * ldH + j] = HT(val[u]);
-        else if (j == i) w.H[(size_t)i * ldH + j] = HT(val[u] + (diag_add ? diag_add[i] : 0.0) + shift);
+        if (j <= i) w.H[(size_t)i * ldH + j] = HT(val[u]);
       }
     }
   }
 }
 
-// H = A + J^T G J + diag(PD + limit + shift), lower triangle, in HT.
-// G at the stored vc per contact; each thread owns one 4x4 tile of H and one
-// of KS slices of the contacts and accumulates J_c^T (G_c J_c) for its tile
-// in registers (G J formed per contact for the tile's columns: no staging,
-// no barriers between contacts); the slices of a tile are summed by warp
-// shuffles (KS a power of two) or add into H in turn, in a fixed order
-// (deterministic).
+// One FP64 tensor-core product: c (8 x 8) += a (8 x 4) b (4 x 8).  Lane l
+// holds a[l / 4][l % 4], b[l % 4][l / 4] and c[l / 4][2 (l % 4) + {0, 1}].
+__device__ __forceinline__ void mma_f64(double& c0, double& c1, double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c0), "+d"(c1)
+      : "d"(a), "d"(b));
+}
+
+// The 8 x 8 blocks of H's lower triangle that a warp forms in one pass: Q0 of
+// block column j0 and Q1 (0 or 1) of block column j1.
+template <int Q0, int Q1>
+struct HessBlocks {
+  int i[Q0 + Q1], j0, j1;  // block rows (past the matrix: nothing to store)
+};
+
+// Adds J^T G J (k steps k0, k0 + dk, ...) to the accumulators of the warp's
+// blocks.  The summed index is the contact row rho = 3 c + r, four rows a
+// step: a = J^T, b = (G J)[rho] = sum_s G[3 rho + s] J[3 c + s] formed on the
+// fly, once per block column.  Rows past 3 count enter with b = 0 (and a read
+// from the last row); block rows and columns past n read the last column and
+// are not stored.
+template <int NT, typename HT, int NS, int Q0, int Q1>
+__device__ __forceinline__ void hess_blocks(const World<NT, HT, NS>& w, const HessBlocks<Q0, Q1>& blk, int k0, int dk,
+                                            double (&acc)[Q0 + Q1][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, l4 = lane & 3;
+  const int n = w.dofs(), ld = w.ldJ(), rows = 3 * w.count;
+  int ca[Q0 + Q1];
+#pragma unroll
+  for (int q = 0; q < Q0 + Q1; ++q) ca[q] = min(8 * blk.i[q] + g, n - 1);
+  const int c0 = min(8 * blk.j0 + g, n - 1), c1 = min(8 * blk.j1 + g, n - 1);
+  const int steps = (rows + 3) / 4;
+#pragma unroll 2
+  for (int k = k0; k < steps; k += dk) {
+    const int rho = 4 * k + l4;
+    const bool live = rho < rows;
+    const int rc = live ? rho : rows - 1;
+    const double* Ja = w.J + rc * ld;
+    const double* Jb = w.J + rc / 3 * 3 * ld;
+    const double* Gr = w.G + 3 * rc;
+    const double g0 = live ? Gr[0] : 0.0, g1 = live ? Gr[1] : 0.0, g2 = live ? Gr[2] : 0.0;
+    const double b0 = g0 * Jb[c0] + g1 * Jb[ld + c0] + g2 * Jb[2 * ld + c0];
+#pragma unroll
+    for (int q = 0; q < Q0; ++q) mma_f64(acc[q][0], acc[q][1], Ja[ca[q]], b0);
+    if (Q1 > 0) {
+      const double b1 = g0 * Jb[c1] + g1 * Jb[ld + c1] + g2 * Jb[2 * ld + c1];
+      mma_f64(acc[Q0 + Q1 - 1][0], acc[Q0 + Q1 - 1][1], Ja[ca[Q0 + Q1 - 1]], b1);
+    }
+  }
+}
+
+// H <- A + J^T G J + diag for the warp's blocks from its accumulators.
+template <int NT, typename HT, int NS, int Q0, int Q1>
+__device__ __forceinline__ void hess_store(const World<NT, HT, NS>& w, const HessBlocks<Q0, Q1>& blk,
+                                           double diag_shift, const double (&acc)[Q0 + Q1][2]) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, l4 = lane & 3;
+  const int n = w.dofs(), ldH = w.ldH();
+#pragma unroll
+  for (int q = 0; q < Q0 + Q1; ++q) {
+    const int i = 8 * blk.i[q] + g, j = 8 * (q < Q0 ? blk.j0 : blk.j1) + 2 * l4;
+    if (i < n && j <= i) {
+      const double* Ai = w.A + i * n + j;
+      HT* Hi = w.H + i * ldH + j;
+      const double hd = w.V(V_HDIAG)[i] + diag_shift;
+      Hi[0] = HT(__ldg(Ai) + acc[q][0] + (i == j ? hd : 0.0));
+      if (j + 1 <= i) Hi[1] = HT(__ldg(Ai + 1) + acc[q][1] + (i == j + 1 ? hd : 0.0));
+    }
+  }
+}
+
+template <int NT, typename HT, int NS, int Q0, int Q1>
+__device__ __forceinline__ void hess_pass(const World<NT, HT, NS>& w, const HessBlocks<Q0, Q1>& blk,
+                                          double diag_shift) {
+  double acc[Q0 + Q1][2];
+#pragma unroll
+  for (int q = 0; q < Q0 + Q1; ++q) acc[q][0] = acc[q][1] = 0.0;
+  hess_blocks<NT, HT, NS, Q0, Q1>(w, blk, 0, 1, acc);
+  hess_store<NT, HT, NS, Q0, Q1>(w, blk, diag_shift, acc);
+}
+
+// H = A + J^T G J + diag(PD + limit + shift), lower triangle, from the
+// derivatives G that evaluate() left: FP64 on the tensor cores
+// (mma.m8n8k4), rounded once to HT.  Register tiles on the FP64 / FP32 cores
+// took 11.6 k / 15.9 k cycles an iteration of 35 DOFs with three / four worlds
+// per SM (20 contacts on average), the FP32 ones converting every element of
+// J at the conversion unit's 16 a cycle.  Whole blocks per warp, so nothing is
+// summed across warps, and the same code on every warp: the blocks are data.
+// (A loop unrolled for each warp's blocks was 2000 instructions, which the
+// instruction cache does not hold beside the rest of the Newton iteration.)
+// 35 DOFs: 15 blocks as four warps' 3 + 1; up to 8 DOFs: the one block's
+// contacts are split over the warps; else passes of one block pair.
 template <int NT, typename HT, int NS>
-__device__ void assemble_hessian(const World<NT, HT, NS>& w, double diag_shift) {
-  const int tid = threadIdx.x;
-  const int n = w.dofs(), ldJ = w.ldJ(), ldH = w.ldH(), nb = w.nb();
-  // G at the current contact velocities (sim/contact_solve.py:1071-1217).
-  for (int c = tid; c < w.count; c += NT) {
-    double g[3], cost, G[9];
-    project_contact(w.cc(c), w.Cn(C_VC + 0)[c], w.Cn(C_VC + 1)[c], w.Cn(C_VC + 2)[c], g, &cost, G);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) w.G[9 * c + k] = HT(G[k]);
-  }
-  // H lower = A lower + diagonal terms
-  load_lower<NT, HT, NS>(w, w.A, w.V(V_HDIAG), diag_shift);
-  const int tiles = nb * (nb + 1) / 2;
-  int ks = NT / (tiles > 0 ? tiles : 1);
-  if (ks < 1) ks = 1;
-  if (ks > 4) ks = 4;
-  const int items = tiles * ks;
-  // This thread's item (a thread holds at most one: items <= NT is checked
-  // on the host; n <= 64 gives tiles <= 136, ks >= 1).
-  const bool has_item = tid < items;
-  int bi = 0, bj = 0, slice = 0;
-  if (has_item) {
-    const int t = tid / ks;
-    slice = tid - t * ks;
-    while ((bi + 1) * (bi + 2) / 2 <= t) ++bi;
-    bj = t - bi * (bi + 1) / 2;
-  }
-  HT acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = HT(0);
-  __syncthreads();  // G ready, H initialised
-  if (has_item) {
-    // this slice's contacts; per contact G J for the tile's 4 columns, then
-    // the tile's rank-3 update J_c[:, 4 bi..]^T (G J_c)[:, 4 bj..]
-    const int per = (w.count + ks - 1) / ks;
-    const int c0 = slice * per, c1 = min(w.count, c0 + per);
-    for (int c = c0; c < c1; ++c) {
-      const double* Jc = w.J + (size_t)(3 * c) * ldJ;
-      HT ja[3][4], jb[3][4], G[9];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          ja[k][q] = HT(Jc[(size_t)k * ldJ + 4 * bi + q]);
-          jb[k][q] = HT(Jc[(size_t)k * ldJ + 4 * bj + q]);
-        }
-#pragma unroll
-      for (int k = 0; k < 9; ++k) G[k] = w.G[9 * c + k];
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        HT gj[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) gj[q] = G[3 * k] * jb[0][q] + G[3 * k + 1] * jb[1][q] + G[3 * k + 2] * jb[2][q];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[a][q] += ja[k][a] * gj[q];
-      }
+__device__ __forceinline__ void assemble_hessian(const World<NT, HT, NS>& w, double diag_shift) {
+  constexpr int NW = NT / 32;
+  const int n = w.dofs(), nb = (n + 7) / 8;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (NS > 0 ? NS <= 8 : nb == 1) {
+    double acc[1][2] = {{0.0, 0.0}};
+    const HessBlocks<1, 0> blk{{0}, 0, 0};
+    const int ks = min(NW, 2 * w.ps / 64);  // the scratch holds one block per warp
+    double* p = w.scr;
+    if (warp < ks) {
+      hess_blocks<NT, HT, NS, 1, 0>(w, blk, warp, ks, acc);
+      p[warp * 64 + 2 * lane] = acc[0][0];
+      p[warp * 64 + 2 * lane + 1] = acc[0][1];
     }
-  }
-  auto add_tile = [&]() {
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const int i = 4 * bi + a;
-      if (i >= n) continue;
-#pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const int j = 4 * bj + b;
-        if (j > i || j >= n) continue;
-        w.H[(size_t)i * ldH + j] += acc[a][b];
-      }
-    }
-  };
-  if ((ks & (ks - 1)) == 0) {
-    // the ks slices of a tile are ks consecutive lanes of one warp: sum them
-    // by shuffles (fixed order), slice 0 adds the tile
-    for (int o = ks >> 1; o > 0; o >>= 1) {
-#pragma unroll
-      for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] += __shfl_down_sync(0xffffffffu, acc[a][b], o);
-    }
-    if (has_item && slice == 0) add_tile();
     __syncthreads();
+    if (warp == 0) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        acc[0][u] = p[2 * lane + u];
+        for (int q = 1; q < ks; ++q) acc[0][u] += p[q * 64 + 2 * lane + u];
+      }
+      hess_store<NT, HT, NS, 1, 0>(w, blk, diag_shift, acc);
+    }
+  } else if constexpr (NT == 128 && NS > 32 && NS <= 40) {
+    // rows warp .. warp + 2 of column `warp`, and the blocks those leave:
+    // (3, 0), (4, 1), (4, 0), (4, 4); warp 3's third row is past the matrix
+    const HessBlocks<3, 1> blk{{warp, warp + 1, warp + 2, warp == 0 ? 3 : 4}, warp,
+                               warp < 2 ? warp : (warp == 2 ? 0 : 4)};
+    hess_pass<NT, HT, NS, 3, 1>(w, blk, diag_shift);
   } else {
-    for (int s = 0; s < ks; ++s) {
-      if (has_item && slice == s) add_tile();
-      __syncthreads();
+    // block pairs (t, t + 1) in row order, (i, j) = row and column of block t
+    const int nblk = nb * (nb + 1) / 2;
+    auto row_of = [](int t) {
+      int i = 0;
+      while ((i + 1) * (i + 2) / 2 <= t) ++i;
+      return i;
+    };
+#pragma unroll 1
+    for (int t = 2 * warp; t < nblk; t += 2 * NW) {
+      const int i0 = row_of(t), i1 = t + 1 < nblk ? row_of(t + 1) : nb;
+      const HessBlocks<1, 1> blk{{i0, i1}, t - i0 * (i0 + 1) / 2, t + 1 < nblk ? t + 1 - i1 * (i1 + 1) / 2 : 0};
+      hess_pass<NT, HT, NS, 1, 1>(w, blk, diag_shift);
     }
   }
+  __syncthreads();
 }
 
 // Newton direction dv = -H^-1 grad: in-place LDL^T of the lower triangle of
 // H (unit L stored below the diagonal unscaled as H_ik = L_ik d_k, D on the
-// diagonal, 1/d_k in V_DINV) by the whole block (ldlt_blocked), then the two
-// triangular solves by warp 0 (ldlt_solve_warp).  Mathematically the
-// Cholesky solve of the reference's BlockCholeskySolverBatched
-// (sim/blocked_cholesky.py:414-604).  (A single-warp factorization measured
-// 3x slower than the block-wide one on 35 x 35: its 35 dependent steps each
-// wait on a shuffle and a shared-memory round trip.  A four-column blocked
-// warp solve measured no faster than the column-by-column one.)  A pivot
-// that is not positive / finite makes dv NaN.
+// diagonal, 1/d_k in V_DINV) by the whole block with -grad carried as row n
+// (its forward substitution is the factorization's own), then the backward
+// substitution by warp 0.  Mathematically the Cholesky solve of the
+// reference's BlockCholeskySolverBatched (sim/blocked_cholesky.py:414-604).
+// A pivot that is not positive / finite makes dv NaN.
 template <int NT, typename HT, int NS, int LB>
-__device__ void factor_and_solve(const World<NT, HT, NS>& w) {
+__device__ __forceinline__ void factor_and_solve(const World<NT, HT, NS>& w) {
   HT* dinv = reinterpret_cast<HT*>(w.V(V_DINV));
-  ldlt_blocked<NT, HT, LB>(w.H, w.dofs(), w.ldH(), dinv, w.tri, w.tri_shift());
+  ldlt_blocked<NT, HT, LB, 1, NS>(w.H, w.dofs(), w.ldH(), dinv, reinterpret_cast<HT*>(w.scr), w.tri, w.tri_shift());
   if ((threadIdx.x >> 5) == 0) {
-    const bool ok = ldlt_pivots_ok_warp<HT>(w.H, w.dofs(), w.ldH());
+    const bool ok = ldlt_backward_warp<HT, NS>(w.H, w.dofs(), w.ldH(), dinv, w.dofs(), w.V(V_DV));
     if (threadIdx.x == 0) *w.factor_ok = ok ? 1 : 0;
-    ldlt_solve_warp<HT>(w.H, w.dofs(), w.ldH(), dinv, w.V(V_GRAD), w.V(V_DV), true, ok);
   }
   __syncthreads();
 }
@@ -441,35 +572,30 @@ __device__ void solve_warp(const World<NT, HT, NS>& w, int rhs_slot, int out_slo
   }
 }
 
-// Line coefficients (sim/contact_solve.py:2234-2263, 1657-1692):
-// dp = A dv, dvc = J dv and {dell0, dell_a0, d2ell_a, mom0}.
+// Line coefficients (sim/contact_solve.py:2234-2263, 1657-1692): dp = A dv,
+// dvc = J dv and warp 0's lanes' shares of {dell0, dell_a0, d2ell_a} (the
+// line search sums them with its first trials).  One barrier: dvc and the
+// partials are then published.
 template <int NT, typename HT, int NS>
-__device__ void line_coefficients(const World<NT, HT, NS>& w, double c4[4]) {
-  const int tid = threadIdx.x;
+__device__ __forceinline__ void line_coefficients(const World<NT, HT, NS>& w, double (&cp)[3]) {
   contact_rows_times<NT, HT, NS>(w, w.V(V_DV), C_DVC);
-  dof_partials<NT, HT, NS>(w, w.V(V_DV), nullptr, false);
+  a_partials<NT, HT, NS>(w, false, false);
   __syncthreads();
-  double d0 = 0.0, da0 = 0.0, d2 = 0.0, m0 = 0.0;
-  const double* v = w.V(V_V);
-  const double* vs = w.V(V_VSTAR);
-  const double* dv = w.V(V_DV);
-  for (int i = tid; i < w.dofs(); i += NT) {
-    const double acc = sum_partials<NT, HT, NS>(w, 0, i);
-    w.V(V_DP)[i] = acc;
-    const double ri = v[i] - vs[i];
-    d0 += w.V(V_GRAD)[i] * dv[i];
-    da0 += acc * ri;
-    d2 += dv[i] * acc;
-    m0 += 0.5 * ri * w.V(V_ARES)[i];
+  cp[0] = cp[1] = cp[2] = 0.0;
+  if (threadIdx.x < 32) {
+#pragma unroll 1
+    for (int i = threadIdx.x; i < w.dofs(); i += 32) {
+      const double acc = sum_partials<NT, HT, NS>(w, 0, i);
+      const double dv = w.V(V_DV)[i];
+      w.V(V_DP)[i] = acc;
+      cp[0] += w.V(V_GRAD)[i] * dv;
+      cp[1] += acc * (w.V(V_V)[i] - w.V(V_VSTAR)[i]);
+      cp[2] += dv * acc;
+    }
   }
-  double r[4] = {d0, da0, d2, m0};
-  block_sum<NT, 4>(r, w.red);  // its barriers also publish dvc / dp
-  c4[0] = r[0];
-  c4[1] = r[1];
-  c4[2] = r[2];
-  c4[3] = r[3];
 }
 
+constexpr int kMixed = -1;  // NS of the kernel that holds every size class's code
 template <int NS> struct LdltBlocks { static constexpr int kCount = 1; static constexpr int kW[1] = {4}; };
 template <> struct LdltBlocks<35> { static constexpr int kCount = 2; static constexpr int kW[2] = {5, 4}; };
 template <> struct LdltBlocks<18> { static constexpr int kCount = 2; static constexpr int kW[2] = {6, 4}; };
@@ -478,8 +604,8 @@ template <> struct LdltBlocks<6> { static constexpr int kCount = 1; static const
 
 // One world of the persistent solve: stage its J and constants, the
 // candidate starts, the Newton loop, the outputs.  NS: the world's DOF count
-// at compile time (0: n_rt at run time); the shared-memory layout L may be
-// sized for more DOFs (n_max) than the world has.
+// at compile time (0: n_rt at run time); the arrays' slots (n_max DOFs) may
+// hold more DOFs than the world has.
 template <int NT, typename HT, int NS, int LSV, int LB>
 __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& L, unsigned char* smem, double* red,
                                             unsigned long long& s_partmask, int& s_factor_ok, const int e,
@@ -487,20 +613,23 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
   const int tid = threadIdx.x;
   const int C = P.p.max_contacts;
   const int n = NS > 0 ? NS : n_rt;
-  World<NT, HT, NS> w{L,
-                  P.p.dynamics_matrix + (size_t)e * n_max * n_max,
-                  reinterpret_cast<double*>(smem + L.off_J),
-                  reinterpret_cast<HT*>(smem + L.off_scr),
-                  reinterpret_cast<HT*>(smem + L.off_H),
-                  reinterpret_cast<HT*>(smem + L.off_G),
-                  reinterpret_cast<double*>(smem + L.off_vec),
-                  reinterpret_cast<double*>(smem + L.off_con),
-                  reinterpret_cast<int*>(smem + L.off_flags),
-                  reinterpret_cast<const uint16_t*>(smem + L.off_tri),
-                  red,
-                  &s_factor_ok,
-                  n,
-                  0};
+  const FixedLayout F = fixed_layout(NS > 0 ? NS : n_max, (int)sizeof(HT), NT);
+  unsigned char* fx = smem + L.off_fixed;
+  World<NT, HT, NS> w{L.n,
+                      F.ps,
+                      P.p.dynamics_matrix + (size_t)e * n_max * n_max,
+                      reinterpret_cast<double*>(smem + L.off_J),
+                      reinterpret_cast<double*>(fx + F.off_scr),
+                      reinterpret_cast<HT*>(fx + F.off_H),
+                      reinterpret_cast<double*>(smem + L.off_G),
+                      reinterpret_cast<double*>(fx + F.off_vec),
+                      reinterpret_cast<double*>(smem + L.off_con),
+                      reinterpret_cast<int*>(fx + F.off_flags),
+                      reinterpret_cast<const uint16_t*>(smem),
+                      red,
+                      &s_factor_ok,
+                      n,
+                      0};
   int count = P.p.contact_count[e];
   if (count > C) count = C;
   if (count < 0) count = 0;
@@ -517,6 +646,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
     // copies (all in flight at once, completed before the barrier after the
     // per-DOF setup below; the rows land at stride ldj).
     const int total = rows * n;
+#pragma unroll 4
     for (int k = tid; k < total; k += NT) {
       const int r = k / n, j = k - r * n;
       const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(w.J + (size_t)r * ldj + j));
@@ -524,24 +654,27 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
     // zero padding columns n..ldj-1
+#pragma unroll 1
     for (int k = tid; k < rows * (ldj - n); k += NT) {
       const int r = k / (ldj - n), j = n + (k - r * (ldj - n));
       w.J[(size_t)r * ldj + j] = 0.0;
     }
+#pragma unroll 1
     for (int c = tid; c < count; c += NT) {
       const size_t ci = (size_t)e * C + c;
       const double tau = P.p.tau_d ? P.p.tau_d[ci] : P.o.contact_tau_d;
       const ContactConst cc = make_contact_const(P.p.phi0[ci], P.p.w_eff[ci], P.p.mu[ci], P.p.stiffness[ci], tau,
                                                  P.o.contact_beta, P.o.contact_sigma, dt);
-      w.Cn(C_RT)[c] = cc.rt;
-      w.Cn(C_RN)[c] = cc.rn;
-      w.Cn(C_RTINV)[c] = cc.rt_inv;
-      w.Cn(C_RNINV)[c] = cc.rn_inv;
-      w.Cn(C_VHAT)[c] = cc.vhat_n;
-      w.Cn(C_MU)[c] = cc.mu;
-      w.Cn(C_MUHAT)[c] = cc.mu_hat;
-      w.Cn(C_FACTOR)[c] = cc.factor;
+      w.cn(c)[C_RT] = cc.rt;
+      w.cn(c)[C_RN] = cc.rn;
+      w.cn(c)[C_RTINV] = cc.rt_inv;
+      w.cn(c)[C_RNINV] = cc.rn_inv;
+      w.cn(c)[C_VHAT] = cc.vhat_n;
+      w.cn(c)[C_MU] = cc.mu;
+      w.cn(c)[C_MUHAT] = cc.mu_hat;
+      w.cn(c)[C_FACTOR] = cc.factor;
     }
+#pragma unroll 1
     for (int i = tid; i < w.ldJ(); i += NT) {
       if (i < n) {
         w.V(V_VSTAR)[i] = P.p.v_star[base + i];
@@ -556,11 +689,12 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
         w.V(V_AINV)[i] = 1.0 / d;
         w.V(V_DSCALE)[i] = 1.0 / sqrt(d);
       } else {
-        for (int k = 0; k < Layout::kVecs; ++k) w.V(k)[i] = 0.0;
+        for (int k = 0; k < kVecs; ++k) w.V(k)[i] = 0.0;
       }
     }
   }
   // ---- PD and limit terms (sim/contact_solve.py:490-683) ------------------
+#pragma unroll 1
   for (int i = tid; i < n; i += NT) {
     int fl = 0;
     const sapb_dof_terms& D = P.dof;
@@ -635,6 +769,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
   // mask in parallel (n <= 60 here).
   if (tid == 0) s_partmask = 0ull;
   __syncthreads();
+#pragma unroll 1
   for (int c = tid; c < count; c += NT) {
     const size_t ci = (size_t)e * C + c;
     unsigned long long mk = 0ull;
@@ -652,12 +787,14 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
     }
     const double* Jc = w.J + (size_t)(3 * c) * w.ldJ();
     if (mk != (1ull << n) - 1ull)
+#pragma unroll 1
       for (int j = 0; j < n; ++j)
         if (Jc[j] != 0.0 || Jc[w.ldJ() + j] != 0.0 || Jc[2 * w.ldJ() + j] != 0.0) mk |= 1ull << j;
     atomicOr(&s_partmask, mk);
   }
   __syncthreads();
   int any_model_term = 0;
+#pragma unroll 1
   for (int i = tid; i < n; i += NT) {
     const int model = (w.flags[i] & (kFlagPd | kFlagLo | kFlagUp)) ? 1 : 0;
     any_model_term |= model;
@@ -667,24 +804,27 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
   const bool unconstrained = (count == 0) && !model_terms;
   // ---- input check: a NaN / Inf in A, J, the contact parameters, v* or
   // the start velocity leaves the world unsolved (SAPB_WORLD_NOT_FINITE)
-  int bad = 0;
-  for (int k = tid; k < n * n; k += NT)
-    if (!isfinite(__ldg(w.A + k))) bad = 1;
+  // (by the exponent bits; J as it lies, padding columns zero)
+  bool bad = false;
+  auto exponent_full = [](int hi) { return (hi & 0x7ff00000) == 0x7ff00000; };
+#pragma unroll 5
+  for (int k = tid; k < n * n; k += NT) bad |= exponent_full(__double2hiint(__ldg(w.A + k)));
   {
-    const int ldj = w.ldJ(), tot = 3 * count * n;
-    for (int k = tid; k < tot; k += NT) {
-      const int r = k / n, j = k - r * n;
-      if (!isfinite(w.J[(size_t)r * ldj + j])) bad = 1;
-    }
+    const int* hi = reinterpret_cast<const int*>(w.J) + 1;
+    const int tot = 3 * count * w.ldJ();
+#pragma unroll 4
+    for (int k = tid; k < tot; k += NT) bad |= exponent_full(hi[2 * k]);
   }
+#pragma unroll 1
   for (int c = tid; c < count; c += NT) {
     const size_t ci = (size_t)e * C + c;
     if (!isfinite(P.p.phi0[ci]) || !isfinite(P.p.w_eff[ci]) || !isfinite(P.p.mu[ci]) ||
         !isfinite(P.p.stiffness[ci]) || (P.p.tau_d && !isfinite(P.p.tau_d[ci])))
-      bad = 1;
+      bad = true;
   }
+#pragma unroll 1
   for (int i = tid; i < n; i += NT)
-    if (!isfinite(w.V(V_VSTAR)[i]) || !isfinite(w.V(V_V)[i])) bad = 1;
+    if (!isfinite(w.V(V_VSTAR)[i]) || !isfinite(w.V(V_V)[i])) bad = true;
   const bool not_finite = __syncthreads_or(bad) != 0;
 
   int newton_iterations = 0, ls_total = 0, converged = 0, status = 0;
@@ -695,9 +835,11 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
     status = SAPB_WORLD_NOT_FINITE;  // v stays the start velocity
   } else if (unconstrained) {
     converged = 1;
+#pragma unroll 1
     for (int i = tid; i < n; i += NT) w.V(V_V)[i] = w.V(V_VSTAR)[i];
     __syncthreads();
   } else {
+#pragma unroll 1
     for (int i = tid; i < n; i += NT)
       if (!(w.flags[i] & kFlagPart)) w.V(V_V)[i] = w.V(V_VSTAR)[i];
     __syncthreads();
@@ -708,125 +850,136 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
     // kernel's factor precision or read from the free motion's factor;
     // the start with the lowest cost among the plain start (unless skipped)
     // and the candidates is taken.  Its evaluation seeds iteration 0 when it
-    // was the last one evaluated.
-    bool have_e4 = false;
-    double e4_seed[4] = {0.0, 0.0, 0.0, 0.0};
+    // was the last one evaluated.  One loop evaluates the starts and the
+    // Newton iterates alike, so the kernel holds one copy of the evaluation.
     const int KV = P.p.v_candidates ? (P.p.v_candidate_count > 1 ? P.p.v_candidate_count : 1) : 0;
     const int KG = P.p.gamma0 ? (P.p.gamma0_count > 1 ? P.p.gamma0_count : 1) : 0;
-    if ((KV > 0 || KG > 0) && count > 0) {
-      // the plain start competes unless the caller skips it; it stays the
-      // fallback when no candidate's cost is finite
-      double best_cost = 1.0e300;
-      if (!P.o.skip_plain_start) {
-        double e4p[4];
-        evaluate<NT, HT, NS>(w, P, dt, e4p);
-        best_cost = e4p[0];
-      }
+    int last_start = KV + KG;  // start 0: the plain one; 1 .. KV: velocities; then the impulse sets
+    int start = -1;            // the start under trial; -1: Newton
+    bool last_is_best = false, zero_sets = false;
+    // the plain start competes unless the caller skips it; it stays the
+    // fallback when no candidate's cost is finite
+    double best_cost = 1.0e300;
+    if (last_start > 0 && count > 0) {
+#pragma unroll 1
       for (int i = tid; i < n; i += NT) w.V(V_SAVE)[i] = w.V(V_V)[i];
-      bool last_is_best = false;
-      auto try_start = [&](int index) {  // V(V_V) holds the candidate
-        __syncthreads();
-        double e4c[4];
-        evaluate<NT, HT, NS>(w, P, dt, e4c);
-        last_is_best = false;
-        if (e4c[0] < best_cost) {
-          best_cost = e4c[0];
-          ws_accepted = index;
-          last_is_best = true;
-          for (int q = 0; q < 4; ++q) e4_seed[q] = e4c[q];
-          for (int i = tid; i < n; i += NT) w.V(V_BEST)[i] = w.V(V_V)[i];
-        }
-      };
-      for (int k = 0; k < KV; ++k) {
-        const double* vk = P.p.v_candidates + ((size_t)k * P.p.num_envs + e) * n_max;
-        for (int i = tid; i < n; i += NT)
-          w.V(V_V)[i] = (w.flags[i] & kFlagPart) ? __ldg(vk + i) : w.V(V_VSTAR)[i];
-        try_start(k + 1);
-      }
-      if (KG > 0) {
-        const double* base_g = P.p.gamma0_base ? P.p.gamma0_base + (size_t)e * n_max : nullptr;
-        // a world whose candidate impulses are all zero starts at the base
-        int nz = 0;
-        for (int q = tid; q < KG * 3 * count; q += NT) {
-          const int kk = q / (3 * count), r = q - kk * 3 * count;
-          if (__ldg(P.p.gamma0 + ((size_t)kk * P.p.num_envs + e) * C * 3 + r) != 0.0) nz = 1;
-        }
-        if (!__syncthreads_or(nz)) {
-          for (int i = tid; i < n; i += NT)
-            w.V(V_V)[i] = (w.flags[i] & kFlagPart) && base_g ? __ldg(base_g + i) : w.V(V_VSTAR)[i];
-          try_start(KV + 1);
-        } else {
-          const int ldj = w.ldJ();
-          if (P.p.dynamics_factor) {
-            // the free motion's LDL^T of A
-            const double* Lg = P.p.dynamics_factor + (size_t)e * n_max * n_max;
-            load_lower<NT, HT, NS>(w, Lg, nullptr, 0.0);
-            HT* dinv = reinterpret_cast<HT*>(w.V(V_DINV));
-            for (int i = tid; i < n; i += NT) dinv[i] = fast_recip(HT(__ldg(Lg + (size_t)i * n + i)));
-            __syncthreads();
-          } else {
-            load_lower<NT, HT, NS>(w, w.A, nullptr, 0.0);
-            __syncthreads();
-            ldlt_blocked<NT, HT, LB>(w.H, n, w.ldH(), reinterpret_cast<HT*>(w.V(V_DINV)), w.tri,
-                                     w.tri_shift());  // the factor of A
-          }
-          // Two sets at a time: stage their impulses in the (here unused)
-          // scratch, form J^T gamma for both (threads 0-63 set k0, 64-127
-          // set k0+1), solve both with the factor on warps 0 and 1, then
-          // evaluate the candidates in order.
-          double* gs = reinterpret_cast<double*>(w.GJ);
-          for (int k0 = 0; k0 < KG; k0 += 2) {
-            const int nk = KG - k0 < 2 ? KG - k0 : 2;
-            for (int q = tid; q < nk * 3 * count; q += NT) {
-              const int kk = q / (3 * count), r = q - kk * 3 * count;
-              gs[q] = __ldg(P.p.gamma0 + ((size_t)(k0 + kk) * P.p.num_envs + e) * C * 3 + r);
-            }
-            __syncthreads();
-            {
-              const int kk = tid >> 6, i = tid & 63;
-              if (kk < nk && i < n) {
-                const double* g = gs + kk * 3 * count;
-                double acc = 0.0;
-                for (int c = 0; c < count; ++c) {
-                  const double* Jc = w.J + (size_t)(3 * c) * ldj;
-                  acc += Jc[i] * g[3 * c] + Jc[ldj + i] * g[3 * c + 1] + Jc[2 * ldj + i] * g[3 * c + 2];
-                }
-                w.V(kk == 0 ? V_GRAD : V_DP)[i] = -acc;  // the solves give -H^-1 rhs
-              }
-            }
-            __syncthreads();
-            solve_warp<NT, HT, NS>(w, V_GRAD, V_DV, 0);
-            if (nk > 1) solve_warp<NT, HT, NS>(w, V_DP, V_DV2, 1);
-            __syncthreads();
-            for (int kk = 0; kk < nk; ++kk) {
-              const double* dvk = w.V(kk == 0 ? V_DV : V_DV2);
-              for (int i = tid; i < n; i += NT)
-                w.V(V_V)[i] = (w.flags[i] & kFlagPart)
-                                  ? (base_g ? __ldg(base_g + i) : w.V(V_VSTAR)[i]) + dvk[i]
-                                  : w.V(V_VSTAR)[i];
-              try_start(KV + k0 + kk + 1);
-            }
-          }
-        }
-      }
-      if (last_is_best) {
-        have_e4 = true;
-      } else {
-        const int src = ws_accepted > 0 ? V_BEST : V_SAVE;
-        for (int i = tid; i < n; i += NT) w.V(V_V)[i] = w.V(src)[i];
-      }
-      __syncthreads();
+      start = P.o.skip_plain_start ? 1 : 0;
     }
     const double cost_min_alpha = LSV == SAPB_LS_MONOTONE_DECAY ? 0.0 : 0.5;
-    int it = 0;
-    bool active = true;
+    int it = 0, from = kEvalFull;
+    bool first = true;
     for (;;) {
-      double e4[4];
-      if (have_e4) {
-        for (int k = 0; k < 4; ++k) e4[k] = e4_seed[k];
-        have_e4 = false;
-      } else {
-        evaluate<NT, HT, NS>(w, P, dt, e4);
+      if (start > 0) {  // V(V_V) <- this start
+        __syncthreads();
+        if (start <= KV) {
+          const double* vk = P.p.v_candidates + ((size_t)(start - 1) * P.p.num_envs + e) * n_max;
+#pragma unroll 1
+          for (int i = tid; i < n; i += NT)
+            w.V(V_V)[i] = (w.flags[i] & kFlagPart) ? __ldg(vk + i) : w.V(V_VSTAR)[i];
+        } else {
+          const double* base_g = P.p.gamma0_base ? P.p.gamma0_base + (size_t)e * n_max : nullptr;
+          const int kg = start - KV - 1;
+          if (kg == 0) {
+            // a world whose candidate impulses are all zero starts at the base
+            int nz = 0;
+#pragma unroll 1
+            for (int q = tid; q < KG * 3 * count; q += NT) {
+              const int kk = q / (3 * count), r = q - kk * 3 * count;
+              if (__ldg(P.p.gamma0 + ((size_t)kk * P.p.num_envs + e) * C * 3 + r) != 0.0) nz = 1;
+            }
+            zero_sets = !__syncthreads_or(nz);
+            if (zero_sets) {
+              last_start = start;
+            } else {
+              HT* dinv = reinterpret_cast<HT*>(w.V(V_DINV));
+              if (P.p.dynamics_factor) {
+                // the free motion's LDL^T of A
+                const double* Lg = P.p.dynamics_factor + (size_t)e * n_max * n_max;
+                load_lower<NT, HT, NS>(w, Lg);
+#pragma unroll 1
+                for (int i = tid; i < n; i += NT) dinv[i] = fast_recip(HT(__ldg(Lg + (size_t)i * n + i)));
+              } else {
+                load_lower<NT, HT, NS>(w, w.A);
+                __syncthreads();
+                ldlt_blocked<NT, HT, LB, 1, 0>(w.H, n, w.ldH(), dinv, reinterpret_cast<HT*>(w.scr), w.tri,
+                                               w.tri_shift());  // the factor of A (row n rides along unread)
+              }
+            }
+          }
+          if (zero_sets) {
+#pragma unroll 1
+            for (int i = tid; i < n; i += NT)
+              w.V(V_V)[i] = (w.flags[i] & kFlagPart) && base_g ? __ldg(base_g + i) : w.V(V_VSTAR)[i];
+          } else {
+            // Two sets at a time: stage their impulses in the place of G (the
+            // next evaluation writes it), form J^T gamma for both (threads 0-63 set kg, 64-127
+            // set kg+1) and solve both with the factor on warps 0 and 1.
+            if (kg % 2 == 0) {
+              const int ldj = w.ldJ();
+              double* gs = w.G;
+              const int nk = KG - kg < 2 ? KG - kg : 2;
+              __syncthreads();
+#pragma unroll 1
+              for (int q = tid; q < nk * 3 * count; q += NT) {
+                const int kk = q / (3 * count), r = q - kk * 3 * count;
+                gs[q] = __ldg(P.p.gamma0 + ((size_t)(kg + kk) * P.p.num_envs + e) * C * 3 + r);
+              }
+              __syncthreads();
+              {
+                const int kk = tid >> 6, i = tid & 63;
+                if (kk < nk && i < n) {
+                  const double* g = gs + kk * 3 * count;
+                  double acc = 0.0;
+#pragma unroll 1
+                  for (int c = 0; c < count; ++c) {
+                    const double* Jc = w.J + (size_t)(3 * c) * ldj;
+                    acc += Jc[i] * g[3 * c] + Jc[ldj + i] * g[3 * c + 1] + Jc[2 * ldj + i] * g[3 * c + 2];
+                  }
+                  w.V(kk == 0 ? V_GRAD : V_DP)[i] = -acc;  // the solves give -H^-1 rhs
+                }
+              }
+              __syncthreads();
+              solve_warp<NT, HT, NS>(w, V_GRAD, V_DV, 0);
+              if (nk > 1) solve_warp<NT, HT, NS>(w, V_DP, V_DP, 1);  // in place
+              __syncthreads();
+            }
+            const double* dvk = w.V(kg % 2 == 0 ? V_DV : V_DP);
+#pragma unroll 1
+            for (int i = tid; i < n; i += NT)
+              w.V(V_V)[i] = (w.flags[i] & kFlagPart) ? (base_g ? __ldg(base_g + i) : w.V(V_VSTAR)[i]) + dvk[i]
+                                                     : w.V(V_VSTAR)[i];
+          }
+        }
+        __syncthreads();
+      }
+      double e4[4], mom;
+      evaluate<NT, HT, NS>(w, P, dt, from, first, alpha, e4, &mom);
+      first = false;
+      if (start >= 0) {
+        if (start == 0) {
+          best_cost = e4[0];
+        } else {
+          last_is_best = e4[0] < best_cost;
+          if (last_is_best) {
+            best_cost = e4[0];
+            ws_accepted = start;
+#pragma unroll 1
+            for (int i = tid; i < n; i += NT) w.V(V_BEST)[i] = w.V(V_V)[i];
+          }
+        }
+        if (start < last_start) {
+          ++start;
+          continue;
+        }
+        start = -1;
+        if (!last_is_best) {
+          __syncthreads();
+          const int src = ws_accepted > 0 ? V_BEST : V_SAVE;
+#pragma unroll 1
+          for (int i = tid; i < n; i += NT) w.V(V_V)[i] = w.V(src)[i];
+          __syncthreads();
+          continue;
+        }
       }
       evaluated = true;
       cost = e4[0];
@@ -844,13 +997,10 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
       newton_iterations = it;
       if (opt || cost_ok) {
         converged = 1;
-        active = false;
-      } else if (it >= P.o.max_iterations) {
-        active = false;
-      } else {
-        converged = 0;
+        break;
       }
-      if (!active) break;
+      if (it >= P.o.max_iterations) break;
+      converged = 0;
       // Newton direction
       assemble_hessian<NT, HT, NS>(w, P.o.diag_shift);
       factor_and_solve<NT, HT, NS, LB>(w);
@@ -860,43 +1010,42 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
         break;
       }
       LsResult r;
-      double c4[4];
-      line_coefficients<NT, HT, NS>(w, c4);
+      double cp[3];
+      line_coefficients<NT, HT, NS>(w, cp);
       if constexpr (LSV == SAPB_LS_ARMIJO_DECAY)
-        r = ls_armijo<NT, 1>(w, P, dt, cost, c4);
+        r = ls_armijo<NT, 1>(w, P, dt, cost, cp, mom);
       else if constexpr (LSV == SAPB_LS_EXACT_ROOT)
-        r = ls_exact<NT>(w, P, dt, cost, c4);
+        r = ls_exact<NT>(w, P, dt, cost, cp, mom);
       else
-        r = ls_monotone<NT, 1>(w, P, dt, cost, c4);
+        r = ls_monotone<NT, 1>(w, P, dt, cost, cp, mom);
       alpha = r.alpha;
       status = r.status;
       constexpr bool mono = LSV == SAPB_LS_MONOTONE_DECAY;
-      if (r.accepted || mono) ls_total += r.iterations;
-      if (r.accepted) {
-        previous_cost = cost;
-        for (int i = tid; i < n; i += NT) w.V(V_V)[i] += r.alpha * w.V(V_DV)[i];
-      } else if (mono) {
+      if (r.accepted || mono) {
+        ls_total += r.iterations;
         previous_cost = cost;
       }
-      __syncthreads();
+      from = r.accepted ? kEvalStep : kEvalSame;
       ++it;
     }
   }
   // ---- outputs ------------------------------------------------------------
+#pragma unroll 1
   for (int i = tid; i < n_max; i += NT) P.out.v[base + i] = i < n ? w.V(V_V)[i] : 0.0;
+#pragma unroll 1
   for (int c = tid; c < C; c += NT) {
     const size_t ci = (size_t)e * C + c;
     const bool live = evaluated && c < count;
     if (P.out.contact_gamma) {
-      P.out.contact_gamma[ci * 3 + 0] = live ? w.Cn(C_GAMMA + 0)[c] : 0.0;
-      P.out.contact_gamma[ci * 3 + 1] = live ? w.Cn(C_GAMMA + 1)[c] : 0.0;
-      P.out.contact_gamma[ci * 3 + 2] = live ? w.Cn(C_GAMMA + 2)[c] : 0.0;
+      P.out.contact_gamma[ci * 3 + 0] = live ? w.cn(c)[C_GAMMA + 0] : 0.0;
+      P.out.contact_gamma[ci * 3 + 1] = live ? w.cn(c)[C_GAMMA + 1] : 0.0;
+      P.out.contact_gamma[ci * 3 + 2] = live ? w.cn(c)[C_GAMMA + 2] : 0.0;
     }
     if (P.out.contact_mode) {
       int mode = SAPB_CONTACT_MODE_NONE;
       if (live) {
         double g[3], cst;
-        mode = project_contact(w.cc(c), w.Cn(C_VC + 0)[c], w.Cn(C_VC + 1)[c], w.Cn(C_VC + 2)[c], g, &cst, nullptr);
+        mode = project_contact(w.cc(c), w.cn(c)[C_VC + 0], w.cn(c)[C_VC + 1], w.cn(c)[C_VC + 2], g, &cst, nullptr);
       }
       P.out.contact_mode[ci] = mode;
     }
@@ -921,18 +1070,24 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
 template <int NT, typename HT, int MINB, int NS, int LSV, int LB>
 __global__ void __launch_bounds__(NT, MINB) contact_solve_kernel(const SolveParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double red[8 * (NT / 32)];
+  __shared__ double red[kRedSize * (NT / 32)];
   __shared__ int s_next;
   __shared__ unsigned long long s_partmask;
   __shared__ int s_factor_ok;
   const int tid = threadIdx.x;
-  // n_max: the DOF slots of a world in the arrays (and the shared-memory
-  // layout); a world's own DOF count may be smaller (dof_count, generic
-  // kernel only), its arrays compact at the start of its slots
-  const int n_max = NS > 0 ? NS : P.p.dof_per_env, C = P.p.max_contacts;
-  const Layout L = make_layout(n_max, C, (int)sizeof(HT), NT / 32);
+  // n_max: the DOF slots of a world in the arrays; a world's own DOF count may
+  // be smaller (dof_count), its arrays compact at the start of its slots
+  const int n_max = P.p.dof_per_env, C = P.p.max_contacts;
+  const Layout L = make_layout(NS > 0 ? NS : n_max, C, (int)sizeof(HT), NT);
   const bool use_guess = P.use_guess_flag_ptr_valid && P.p.v_guess_active[0] != 0;
-  build_triangle_list<NT>(reinterpret_cast<uint16_t*>(smem + L.off_tri), n_max);
+  build_triangle_list<NT>(reinterpret_cast<uint16_t*>(smem), L.n, 1);
+  // the DOFs of world e, and whether it is this launch's
+  auto dofs_of = [&](int e) {
+    if (!P.p.dof_count) return n_max;
+    const int d = P.p.dof_count[e];
+    return d < 1 ? 1 : (d > n_max ? n_max : d);
+  };
+  auto takes = [&](int d) { return !P.own_class_only || (NS > 0 ? d == NS : !specialised_dofs(d)); };
 
   if (tid == 0) s_next = atomicAdd(P.queue, 1);
   for (;;) {
@@ -946,10 +1101,12 @@ __global__ void __launch_bounds__(NT, MINB) contact_solve_kernel(const SolvePara
     if (tid == 0) s_next = atomicAdd(P.queue, 1);
     __syncthreads();
     if (e < 0 || e >= P.p.num_envs) continue;
+    const int n_world = dofs_of(e);
+    if (!takes(n_world)) continue;
     {
       const int nt = s_next;
       const int nx = nt < P.p.num_envs ? (P.p.world_order ? P.p.world_order[nt] : nt) : P.p.num_envs;
-      if (nx >= 0 && nx < P.p.num_envs) {
+      if (nx >= 0 && nx < P.p.num_envs && takes(dofs_of(nx))) {
         const char* a0 = reinterpret_cast<const char*>(P.p.dynamics_matrix + (size_t)nx * n_max * n_max);
         const size_t abytes = sizeof(double) * (size_t)n_max * n_max;
         int cnt = P.p.contact_count[nx];
@@ -987,43 +1144,30 @@ __global__ void __launch_bounds__(NT, MINB) contact_solve_kernel(const SolvePara
       }
     }
 
-    int n_world = n_max;
-    if (NS == 0 && P.p.dof_count) {
-      n_world = P.p.dof_count[e];
-      n_world = n_world < 1 ? 1 : (n_world > n_max ? n_max : n_world);
-    }
-    if constexpr (NS == 0) {
-      if (P.p.dof_count) {
-        // each world's own DOF count: the specialised code of its size class
-        switch (n_world) {
-          case 35:
-            solve_world<NT, HT, 35, LSV, LdltBlocks<35>::kW[0]>(P, L, smem, red, s_partmask, s_factor_ok, e,
-                                                                 n_max, 35, use_guess);
-            continue;
-          case 18:
-            solve_world<NT, HT, 18, LSV, LdltBlocks<18>::kW[0]>(P, L, smem, red, s_partmask, s_factor_ok, e,
-                                                                 n_max, 18, use_guess);
-            continue;
-          case 13:
-            solve_world<NT, HT, 13, LSV, LdltBlocks<13>::kW[0]>(P, L, smem, red, s_partmask, s_factor_ok, e,
-                                                                 n_max, 13, use_guess);
-            continue;
-          case 6:
-            solve_world<NT, HT, 6, LSV, LdltBlocks<6>::kW[0]>(P, L, smem, red, s_partmask, s_factor_ok, e,
-                                                                 n_max, 6, use_guess);
-            continue;
-          default:
-            break;
-        }
+    if constexpr (NS == kMixed) {
+      // each world's own DOF count: the specialised code of its size class
+#define SAPB_CLASS(N)                                                                                              \
+  case N:                                                                                                          \
+    solve_world<NT, HT, N, LSV, LdltBlocks<N>::kW[0]>(P, L, smem, red, s_partmask, s_factor_ok, e, n_max, N, use_guess); \
+    break;
+      switch (n_world) {
+        SAPB_CLASS(35)
+        SAPB_CLASS(18)
+        SAPB_CLASS(13)
+        SAPB_CLASS(6)
+        default:
+          solve_world<NT, HT, 0, LSV, LB>(P, L, smem, red, s_partmask, s_factor_ok, e, n_max, n_world, use_guess);
       }
+#undef SAPB_CLASS
+    } else {
+      solve_world<NT, HT, NS, LSV, LB>(P, L, smem, red, s_partmask, s_factor_ok, e, n_max, n_world, use_guess);
     }
-    solve_world<NT, HT, NS, LSV, LB>(P, L, smem, red, s_partmask, s_factor_ok, e, n_max, n_world, use_guess);
   }
 }
 
 template <int NT, typename HT, int MINB, int NS, int LSV, int LB>
 cudaError_t launch_solve_ls(const SolveParams& P, cudaStream_t stream, int* blocks_out) {
-  const Layout L = make_layout(P.p.dof_per_env, P.p.max_contacts, (int)sizeof(HT), NT / 32);
+  const Layout L = make_layout(NS > 0 ? NS : P.p.dof_per_env, P.p.max_contacts, (int)sizeof(HT), NT);
   auto kern = contact_solve_kernel<NT, HT, MINB, NS, LSV, LB>;
   cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
   if (err != cudaSuccess) return err;
@@ -1046,8 +1190,6 @@ cudaError_t launch_solve_ls(const SolveParams& P, cudaStream_t stream, int* bloc
   if (blocks > P.p.num_envs) blocks = P.p.num_envs;
   if (blocks < 1) blocks = 1;
   if (blocks_out) *blocks_out = blocks;
-  err = cudaMemsetAsync(P.queue, 0, sizeof(int32_t), stream);
-  if (err != cudaSuccess) return err;
   kern<<<blocks, NT, L.total, stream>>>(P);
   return cudaGetLastError();
 }
@@ -1103,10 +1245,12 @@ extern template cudaError_t launch_solve_wide<false>(const SolveParams&, cudaStr
 
 // The runtime-size kernels (128 and 256 threads) are the largest: each line
 // search's kernel is instantiated in a translation unit of its own
-// (sapb_solve_n{generic,wide}_f{32,64}_{armijo,exact,monotone}.cu).
+// (sapb_solve_n{generic,mixed,wide}_f{32,64}_{armijo,exact,monotone}.cu).
 #define SAPB_RUNTIME_SIZE_KERNELS(X, LSV)                                         \
   X(128, float, 4, 0, LSV, LdltBlocks<0>::kW[0])                                \
   X(128, double, 3, 0, LSV, LdltBlocks<0>::kW[0])                               \
+  X(128, float, 4, kMixed, LSV, LdltBlocks<0>::kW[0])                           \
+  X(128, double, 3, kMixed, LSV, LdltBlocks<0>::kW[0])                          \
   X(256, float, 2, 0, LSV, LdltBlocks<0>::kW[0])                                \
   X(256, double, 1, 0, LSV, LdltBlocks<0>::kW[0])
 #define SAPB_EXTERN_LS(NT, HT, MINB, NS, LSV, LB) \
@@ -1124,6 +1268,7 @@ SAPB_EXTERN_SOLVE(18)
 SAPB_EXTERN_SOLVE(13)
 SAPB_EXTERN_SOLVE(6)
 SAPB_EXTERN_SOLVE(0)
+SAPB_EXTERN_SOLVE(kMixed)
 #undef SAPB_EXTERN_SOLVE
 
 }  // namespace sapb

@@ -60,8 +60,12 @@ __device__ __forceinline__ int project_contact(const ContactConst& cc, double vc
   const double y1 = -cc.rt_inv * vcy;
   const double y2 = cc.rn_inv * (cc.vhat_n - vcz);
   const double m = cc.mu;
-  const double yr = sqrt(y0 * y0 + y1 * y1 + kSoftNormTol * kSoftNormTol);
-  const double inv_yr = 1.0 / yr;  // yr >= 1e-7 > 0
+  // the soft norm and its reciprocal from one reciprocal square root (one
+  // correction step for the norm), not a square root and a division
+  const double yy = y0 * y0 + y1 * y1 + kSoftNormTol * kSoftNormTol;  // >= 1e-14 > 0
+  const double inv_yr = rsqrt(yy);
+  double yr = yy * inv_yr;
+  yr = fma(fma(-yr, yr, yy), 0.5 * inv_yr, yr);
   const double tx = y0 * inv_yr, ty = y1 * inv_yr;
   double g0 = 0.0, g1 = 0.0, g2 = 0.0;
   int mode = SAPB_CONTACT_MODE_NONE;
@@ -88,7 +92,7 @@ __device__ __forceinline__ int project_contact(const ContactConst& cc, double vc
         G[8] = cc.rn_inv;
       }
       mode = SAPB_CONTACT_MODE_STICTION;
-    } else if ((-mu_hat * yr < y2) && (y2 < yr / m)) {
+    } else if (-mu_hat * yr < y2) {  // (and y2 < yr / m, the converse of stiction)
       const double gn = (y2 + mu_hat * yr) * factor;
       g0 = m * gn * tx;
       g1 = m * gn * ty;
@@ -191,6 +195,20 @@ __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
+}
+
+// Sums of four values over a warp in six exchanges: halves of the lanes keep
+// two of them, quarters one.  Lane 8 k (and the seven after it) return the sum
+// of the k-th.
+__device__ __forceinline__ double warp_sum4(double v0, double v1, double v2, double v3) {
+  const int lane = threadIdx.x & 31;
+  const bool hi = lane & 16, odd = lane & 8;
+  const double a0 = (hi ? v2 : v0) + __shfl_xor_sync(0xffffffffu, hi ? v0 : v2, 16);
+  const double a1 = (hi ? v3 : v1) + __shfl_xor_sync(0xffffffffu, hi ? v1 : v3, 16);
+  double a = (odd ? a1 : a0) + __shfl_xor_sync(0xffffffffu, odd ? a0 : a1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
 }
 
 // Sum K values over the block; every thread receives the totals.  `red` is a

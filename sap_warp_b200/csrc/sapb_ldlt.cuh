@@ -5,114 +5,254 @@
 #pragma once
 
 #include <cstdint>
+#include <type_traits>
 
 #include "sapb_device.cuh"
 
 namespace sapb {
 
-// Column-descending list of the lower triangle below row 0: entries
-// (i << 8 | j) for j = n-1 .. 1, i = j .. n-1.  The trailing triangle of
-// columns > k is its first m(m+1)/2 entries, m = n-1-k.  n <= 256.
+// Column-descending list of the lower triangle below row 0, each column
+// followed by its nrhs right-hand-side rows: entries (i << 8 | j) for j = n-1
+// .. 1, i = j .. n-1+nrhs.  The trailing triangle of columns > k is its first
+// m(m+1)/2 + nrhs m entries, m = n-1-k.  n + nrhs <= 256.
+__host__ __device__ constexpr int triangle_list_size(int n, int nrhs) {
+  return n * (n - 1) / 2 + nrhs * (n - 1) + 1;
+}
 template <int NT>
-__device__ __forceinline__ void build_triangle_list(uint16_t* tri, int n) {
+__device__ __forceinline__ void build_triangle_list(uint16_t* tri, int n, int nrhs) {
+#pragma unroll 1
   for (int j = n - 1 - (int)threadIdx.x; j >= 1; j -= NT) {
-    const int off = (n - 1 - j) * (n - j) / 2;
-    for (int i = j; i < n; ++i) tri[off + (i - j)] = (uint16_t)((i << 8) | j);
+    const int m = n - 1 - j;
+    const int off = m * (m + 1) / 2 + nrhs * m;
+    for (int i = j; i < n + nrhs; ++i) tri[off + (i - j)] = (uint16_t)((i << 8) | j);
+  }
+}
+
+// Pivot reciprocal of the factorization: Newton-Raphson steps from the
+// hardware's approximation (two in FP64, one in FP32), without a range check:
+// a pivot that is not positive and finite, or beyond the reciprocal's range,
+// gives one that is not, and is reported by it (ldlt_backward_warp,
+// ldlt_pivots_ok_warp).
+__device__ __forceinline__ double pivot_recip(double d) {
+  double x;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
+  x = fma(x, fma(-d, x, 1.0), x);
+  return fma(x, fma(-d, x, 1.0), x);
+}
+__device__ __forceinline__ float pivot_recip(float d) {
+  float x;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(d));
+  return fmaf(x, fmaf(-d, x, 1.0f), x);
+}
+
+// Values of S (the scaled panel) per row: B rounded up so that rows are
+// 16-byte aligned.
+template <typename T, int B>
+__host__ __device__ constexpr int ldlt_panel_stride() {
+  return sizeof(T) == 8 ? (B + 1) / 2 * 2 : (B + 3) / 4 * 4;
+}
+
+// The B values of a row of S, 16 bytes at a time.
+template <typename T, int B>
+__device__ __forceinline__ void load_panel_row(const T* Sj, T (&v)[B]) {
+  constexpr int V = 16 / sizeof(T);
+  using V16 = typename std::conditional<sizeof(T) == 8, double2, float4>::type;
+#pragma unroll
+  for (int c = 0; c < B; c += V) {
+    const V16 q = *reinterpret_cast<const V16*>(Sj + c);
+    const T* e = reinterpret_cast<const T*>(&q);
+#pragma unroll
+    for (int u = 0; u < V; ++u)
+      if (c + u < B) v[c + u] = e[u];
   }
 }
 
 // In-place right-looking LDL^T of the lower triangle of H (row stride ldH;
-// tri: the triangle list of build_triangle_list for n + tri_shift DOFs):
-// afterwards H_ik = L_ik d_k below the diagonal (L unit lower), d_k on it,
-// dinv[k] = 1/d_k.  B-column blocks, two barriers per block:
-// every thread factors the block's diagonal block in
-// registers (it is final once the previous trailing update is done), the rows
-// under it (the panel) are solved against it in registers, one per thread;
-// after the panel's barrier threads below bs write the block's rows back
-// while the trailing update runs.  The arithmetic is the right-looking
+// tri: the triangle list of build_triangle_list for n + tri_shift DOFs and
+// NRHS right-hand sides): afterwards H_ik = L_ik d_k below the diagonal (L
+// unit lower), d_k on it, dinv[k] = 1/d_k.  NRHS: H holds that many more rows
+// from n on, right-hand sides b; they are carried through the panels like any
+// other row and end as L^-1 b, so the forward substitution costs no pass of
+// its own.  NS: n at compile time, or 0.
+//
+// B-column blocks, two barriers per block.  Panel: every thread that holds a
+// row below the block eliminates it against the block's B x B diagonal block,
+// which it factors in registers (its own copy: a shuffle costs more than the
+// arithmetic).  Trailing triangle: every thread owns the same entries of the
+// list throughout -- the prefix that is left only shrinks -- and with NS
+// keeps them in registers until their column's panel is next; the panel is
+// read as B-value rows, unscaled from H, divided by the pivots and negated
+// from S.  A world's whole time here is latency: about 100 dependent
+// instructions of one warp a panel.  The arithmetic is the right-looking
 // recurrence on the stored form W_ik = L_ik d_k:
 //   d_k = H_kk - sum_{e<k} W_ke^2 / d_e,  W_ik = H_ik - sum_{e<k} W_ie W_ke / d_e.
-// H must be complete when called (barrier before); complete on return.
-template <int NT, typename T, int B>
-__device__ void ldlt_blocked(T* H, int n, int ldH, T* dinv, const uint16_t* tri, int tri_shift = 0) {
+// H must be complete when called (barrier before); complete on return (NRHS:
+// to warp 0; the last block's rows are its alone).
+template <int NT, typename T, int B, int NRHS, int NS>
+__device__ __forceinline__ void ldlt_blocked(T* H, int n, int ldH, T* dinv, T* S, const uint16_t* tri,
+                                             int tri_shift = 0) {
   static_assert(B >= 1 && B <= 8, "block width");
+  constexpr int kS = ldlt_panel_stride<T, B>();
+  constexpr int kLeft = NS > B ? NS - B : 0;  // columns right of the first block
+  constexpr int kRounds = NS > 0 ? (kLeft * (kLeft + 1) / 2 + NRHS * kLeft + NT - 1) / NT : 0;
+  constexpr bool kWhole = NS > 0 && NS % B == 0;  // no partial block
   const int tid = threadIdx.x;
+  const int rows = n + NRHS;
+  T acc[kRounds > 0 ? kRounds : 1];
+  int at[kRounds > 0 ? kRounds : 1];  // i << 8 | j, -1: no entry
+  if constexpr (kRounds > 0) {
+    const int left = n - B, cnt = left > 0 ? left * (left + 1) / 2 + NRHS * left : 0;
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int e = tid + r * NT;
+      at[r] = e < cnt ? (int)tri[e] - tri_shift * 257 : -1;
+      acc[r] = e < cnt ? H[(at[r] >> 8) * ldH + (at[r] & 255)] : T(0);
+    }
+  }
+#pragma unroll 1
   for (int K = 0; K < n; K += B) {
-    const int bs = min(B, n - K);
-    const int rest = n - K - bs;
-    // (1) the diagonal block, in registers (padding rows: identity)
+    const int bs = kWhole ? B : min(B, n - K);
+    const int rest = n - K - bs, prow = rows - K - bs;
     T W[B][B], R[B];
+    if ((tid & ~31) < (prow > 1 ? prow : 1)) {
+      // the diagonal block (padding rows: identity)
+      const T* Hd = H + K * ldH + K;
 #pragma unroll
-    for (int a = 0; a < B; ++a)
+      for (int a = 0; a < B; ++a)
 #pragma unroll
-      for (int b = 0; b <= a; ++b)
-        W[a][b] = (a < bs) ? H[(size_t)(K + a) * ldH + K + b] : (a == b ? T(1) : T(0));
-#pragma unroll
-    for (int b = 0; b < B; ++b) {
-      T d = W[b][b];
-#pragma unroll
-      for (int e = 0; e < b; ++e) d -= W[b][e] * R[e] * W[b][e];
-      W[b][b] = d;
-      R[b] = fast_recip(d);
-#pragma unroll
-      for (int a = b + 1; a < B; ++a) {
-        T v = W[a][b];
-#pragma unroll
-        for (int e = 0; e < b; ++e) v -= W[a][e] * R[e] * W[b][e];
-        W[a][b] = v;
-      }
-    }
-    // The factored rows go back to H only once every thread has read the
-    // block: after the panel's barrier (the trailing update never touches
-    // the diagonal block), or after a barrier of its own for the last block.
-    auto store_block = [&]() {
-      if (tid < bs) {
-#pragma unroll
-        for (int a = 0; a < B; ++a) {
-          if (a != tid) continue;
-#pragma unroll
-          for (int b = 0; b <= a; ++b) H[(size_t)(K + a) * ldH + K + b] = W[a][b];
-          dinv[K + a] = R[a];
-        }
-      }
-    };
-    if (rest <= 0) {
-      __syncthreads();
-      store_block();
-      __syncthreads();
-      break;
-    }
-    // (2) panel rows: P L_K^T = H_panel (forward substitution over the block columns)
-    for (int t = tid; t < rest; t += NT) {
-      const int i = K + bs + t;
-      T p[B];
+        for (int b = 0; b <= a; ++b) W[a][b] = a < bs ? Hd[a * ldH + b] : (a == b ? T(1) : T(0));
 #pragma unroll
       for (int c = 0; c < B; ++c) {
-        if (c < bs) {
-          T h = H[(size_t)i * ldH + K + c];
+        R[c] = pivot_recip(W[c][c]);
 #pragma unroll
-          for (int m2 = 0; m2 < c; ++m2) h -= p[m2] * (W[c][m2] * R[m2]);
-          p[c] = h;
-          H[(size_t)i * ldH + K + c] = h;
+        for (int m = c + 1; m < B; ++m) {
+          const T l = W[m][c] * R[c];
+#pragma unroll
+          for (int m2 = c + 1; m2 <= m; ++m2) W[m][m2] -= l * W[m2][c];
         }
       }
+      auto eliminate = [&](int t) {
+        const int i = K + bs + t;
+        T* Hi = H + i * ldH + K;
+        T v[B], q[B];
+#pragma unroll
+        for (int c = 0; c < B; ++c) v[c] = c < bs ? Hi[c] : T(0);
+#pragma unroll
+        for (int c = 0; c < B; ++c) {
+          q[c] = -v[c] * R[c];
+#pragma unroll
+          for (int m = c + 1; m < B; ++m) v[m] += q[c] * W[m][c];
+        }
+        T* Si = S + (i < n ? i : n) * kS;  // (right-hand sides: a row past the others, not read)
+#pragma unroll
+        for (int c = 0; c < B; ++c)
+          if (c < bs) {
+            Hi[c] = v[c];
+            Si[c] = q[c];
+          }
+      };
+      if constexpr (NS > 0) {  // every row has its thread
+        if (tid < prow) eliminate(tid);
+      } else {
+#pragma unroll 1
+        for (int t = tid; t < prow; t += NT) eliminate(t);
+      }
+    }
+    // The factored block goes back to H once every thread has read it: at
+    // once when one warp holds all panel rows, else after the panel's barrier
+    // (the trailing update never touches the diagonal block).  Every lane of
+    // warp 0 holds the same values and stores them all: no selection by lane.
+    const bool one_warp = prow <= 32;
+    auto store_block = [&]() {
+#pragma unroll
+      for (int a = 0; a < B; ++a)
+        if (a < bs) {
+#pragma unroll
+          for (int b = 0; b <= a; ++b) H[(K + a) * ldH + K + b] = W[a][b];
+          dinv[K + a] = R[a];
+        }
+    };
+    if (one_warp && tid < 32) {
+      __syncwarp();
+      store_block();
+    }
+    if (rest <= 0) {
+      if (NRHS > 0) __syncwarp();
+      else __syncthreads();
+      break;
     }
     __syncthreads();
-    store_block();
-    // (3) trailing update of entries (i, j), j >= K + bs: the first
-    // rest*(rest+1)/2 entries of the column-descending triangle list.
-    const int cnt = rest * (rest + 1) / 2;
-    for (int e = tid; e < cnt; e += NT) {
-      const int ij = tri[e];
-      const int i = (ij >> 8) - tri_shift, j = (ij & 255) - tri_shift;
-      T acc = H[(size_t)i * ldH + j];
+    if (!one_warp && tid < 32) store_block();
+    // trailing update of entries (i, j), j >= K + bs: the first entries of
+    // the column-descending list
+    const int cnt = rest * (rest + 1) / 2 + NRHS * rest;
+    const T* Hk = H + K;
+    if constexpr (kRounds > 0) {
 #pragma unroll
-      for (int c = 0; c < B; ++c)
-        if (c < bs) acc -= H[(size_t)i * ldH + K + c] * R[c] * H[(size_t)j * ldH + K + c];
-      H[(size_t)i * ldH + j] = acc;
+      for (int r = 0; r < kRounds; ++r) {
+        if (r * NT < cnt) {
+          const int e = tid + r * NT;
+          const int i = at[r] >> 8, j = at[r] & 255;
+          if (e < cnt) {
+            const T* Hi = Hk + i * ldH;
+            T sj[B];
+            load_panel_row<T, B>(S + j * kS, sj);
+#pragma unroll
+            for (int c = 0; c < B; ++c) acc[r] += Hi[c] * sj[c];
+            if (j < K + 2 * B) H[i * ldH + j] = acc[r];  // its column is next
+          }
+        }
+      }
+    } else {
+#pragma unroll 2
+      for (int e = tid; e < cnt; e += NT) {
+        const int ij = tri[e] - tri_shift * 257;
+        const int i = ij >> 8, j = ij & 255;
+        T* h = H + i * ldH + j;
+        const T* Hi = Hk + i * ldH;
+        T sj[B];
+        load_panel_row<T, B>(S + j * kS, sj);
+        T v = *h;
+#pragma unroll
+        for (int c = 0; c < B; ++c) v += Hi[c] * sj[c];
+        *h = v;
+      }
     }
     __syncthreads();
   }
+}
+
+// x = L^-T D^-1 y by the calling warp alone, y = row `rhs` of the LDL^T that
+// ldlt_blocked left in H: lanes own rows lane and lane + 32 (n <= 64) and
+// hold z = (y - sum_{k > i} W_ki x_k) / d; from the last row on, x_k = z_k
+// goes round by a shuffle.  Bound by the chain of a shuffle and a fused
+// multiply-add a row.  Returns, to every lane, whether every pivot is
+// positive and finite (by its reciprocal); if not, x is NaN.
+template <typename T, int NS>
+__device__ __forceinline__ bool ldlt_backward_warp(const T* H, int n, int ldH, const T* dinv, int rhs, double* x) {
+  const int lane = threadIdx.x & 31;
+  const T* y = H + rhs * ldH;
+  const T d0 = lane < n ? dinv[lane] : T(1), d1 = lane + 32 < n ? dinv[lane + 32] : T(1);
+  const bool ok = __all_sync(0xffffffffu, d0 > T(0) && d0 < T(INFINITY) && d1 > T(0) && d1 < T(INFINITY));
+  T z0 = lane < n ? y[lane] * d0 : T(0), z1 = lane + 32 < n ? y[lane + 32] * d1 : T(0);
+  const T* Hl = H + lane;
+  int k = n - 1;
+#pragma unroll 1
+  for (; k >= 32; --k) {  // rows of the second slot
+    const T w0 = Hl[k * ldH] * d0, w1 = lane + 32 < k ? Hl[k * ldH + 32] * d1 : T(0);
+    const T xk = __shfl_sync(0xffffffffu, z1, k - 32);
+    z1 -= w1 * xk;
+    z0 -= w0 * xk;
+  }
+#pragma unroll 4
+  for (; k > 0; --k) {
+    const T w0 = lane < k ? Hl[k * ldH] * d0 : T(0);
+    z0 -= w0 * __shfl_sync(0xffffffffu, z0, k);
+  }
+  const double nanv = __longlong_as_double(0x7ff8000000000000ULL);
+  if (lane < n) x[lane] = ok ? double(z0) : nanv;
+  if (lane + 32 < n) x[lane + 32] = ok ? double(z1) : nanv;
+  return ok;
 }
 
 // x <- -A^-1 x (neg) or A^-1 x with the LDL^T that ldlt_blocked left in H
@@ -215,6 +355,7 @@ __device__ void ldlt_solve_warp(const T* H, int n, int ldH, const T* dinv, const
   const T sg = neg ? T(-1) : T(1);
   T h0 = lane < n ? sg * T(b[lane]) : T(0);
   T h1 = lane + 32 < n ? sg * T(b[lane + 32]) : T(0);
+#pragma unroll 1
   for (int k = 0; k < n; ++k) {
     const T zk = __shfl_sync(0xffffffffu, k < 32 ? h0 : h1, k & 31) * dinv[k];
     if (lane == (k & 31)) {
@@ -225,6 +366,7 @@ __device__ void ldlt_solve_warp(const T* H, int n, int ldH, const T* dinv, const
     if (lane + 32 > k && lane + 32 < n) h1 -= H[(size_t)(lane + 32) * ldH + k] * zk;
   }
   T s0 = T(0), s1 = T(0);
+#pragma unroll 1
   for (int i = n - 1; i >= 0; --i) {
     T xi_local = T(0);
     if (lane == (i & 31)) {

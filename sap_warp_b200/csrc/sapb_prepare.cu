@@ -258,6 +258,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   double* adiag = tau + 2 * n;
   double* dinv = tau + 3 * n;
   double* H = reinterpret_cast<double*>(smem + L.H);
+  double* pan = Fi;  // the factor's scaled panel: 6 a row, once A is formed from F
   double* con = reinterpret_cast<double*>(smem + L.con);
   int* conint = reinterpret_cast<int*>(smem + L.conint);
   uint64_t* ancA = reinterpret_cast<uint64_t*>(smem + L.anc);
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     if (blk) btree[b] = -1;
   }
   for (int i = tid; i < n; i += kPrepNT) dbody[i] = -1;
-  if (!blk) build_triangle_list<kPrepNT>(tri, n);
+  if (!blk) build_triangle_list<kPrepNT>(tri, n, 0);
   for (int k = tid; k < 6 * n; k += kPrepNT) S[k] = 0.0;
   if (want_vstart)
     for (int k = tid; k < (kPrepNT / 32) * n; k += kPrepNT) jg[k] = 0.0;
@@ -665,7 +666,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
       }
     }
   } else {
-  ldlt_blocked<kPrepNT, double, 5>(H, n, n, dinv, tri);  // width 5: measured fastest for 35 DOFs
+  ldlt_blocked<kPrepNT, double, 5, 0, 0>(H, n, n, dinv, pan, tri);  // width 5: measured fastest for 35 DOFs
   if (write_factor) {
     double* Lg = P.out.dynamics_factor + (size_t)e * n_slot * n_slot;
     for (int k = tid; k < n * n; k += kPrepNT) {

@@ -1,4 +1,4 @@
-// Contact-solve kernels sized at run time (n <= 60; with per-world DOF counts each world runs the code of its size class); FP64 Hessian and factor.
+// Contact-solve kernels sized at run time (n <= 60); FP64 Hessian and factor.
 #include "sapb_contact_solve.cuh"
 
 namespace sapb {
