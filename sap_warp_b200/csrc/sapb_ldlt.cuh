@@ -222,19 +222,12 @@ __device__ __forceinline__ void ldlt_blocked(T* H, int n, int ldH, T* dinv, T* S
   }
 }
 
-// x = L^-T D^-1 y by the calling warp alone, y = row `rhs` of the LDL^T that
-// ldlt_blocked left in H: lanes own rows lane and lane + 32 (n <= 64) and
-// hold z = (y - sum_{k > i} W_ki x_k) / d; from the last row on, x_k = z_k
-// goes round by a shuffle.  Bound by the chain of a shuffle and a fused
-// multiply-add a row.  Returns, to every lane, whether every pivot is
-// positive and finite (by its reciprocal); if not, x is NaN.
-template <typename T, int NS>
-__device__ __forceinline__ bool ldlt_backward_warp(const T* H, int n, int ldH, const T* dinv, int rhs, double* x) {
+// z <- L^-T z by the calling warp: lanes hold z of rows lane and lane + 32
+// (n <= 64) and their d0, d1 = 1/d.  From the last row on, x_k = z_k goes round
+// by a shuffle: a chain of a shuffle and a fused multiply-add a row.
+template <typename T>
+__device__ __forceinline__ void ldlt_backward_lanes(const T* H, int n, int ldH, T d0, T d1, T& z0, T& z1) {
   const int lane = threadIdx.x & 31;
-  const T* y = H + rhs * ldH;
-  const T d0 = lane < n ? dinv[lane] : T(1), d1 = lane + 32 < n ? dinv[lane + 32] : T(1);
-  const bool ok = __all_sync(0xffffffffu, d0 > T(0) && d0 < T(INFINITY) && d1 > T(0) && d1 < T(INFINITY));
-  T z0 = lane < n ? y[lane] * d0 : T(0), z1 = lane + 32 < n ? y[lane + 32] * d1 : T(0);
   const T* Hl = H + lane;
   int k = n - 1;
 #pragma unroll 1
@@ -249,6 +242,19 @@ __device__ __forceinline__ bool ldlt_backward_warp(const T* H, int n, int ldH, c
     const T w0 = lane < k ? Hl[k * ldH] * d0 : T(0);
     z0 -= w0 * __shfl_sync(0xffffffffu, z0, k);
   }
+}
+
+// x = L^-T D^-1 y by the calling warp alone, y = row `rhs` of the LDL^T that
+// ldlt_blocked left in H (n <= 64).  Returns, to every lane, whether every
+// pivot is positive and finite (by its reciprocal); if not, x is NaN.
+template <typename T, int NS>
+__device__ __forceinline__ bool ldlt_backward_warp(const T* H, int n, int ldH, const T* dinv, int rhs, double* x) {
+  const int lane = threadIdx.x & 31;
+  const T* y = H + rhs * ldH;
+  const T d0 = lane < n ? dinv[lane] : T(1), d1 = lane + 32 < n ? dinv[lane + 32] : T(1);
+  const bool ok = __all_sync(0xffffffffu, d0 > T(0) && d0 < T(INFINITY) && d1 > T(0) && d1 < T(INFINITY));
+  T z0 = lane < n ? y[lane] * d0 : T(0), z1 = lane + 32 < n ? y[lane + 32] * d1 : T(0);
+  ldlt_backward_lanes(H, n, ldH, d0, d1, z0, z1);
   const double nanv = __longlong_as_double(0x7ff8000000000000ULL);
   if (lane < n) x[lane] = ok ? double(z0) : nanv;
   if (lane + 32 < n) x[lane + 32] = ok ? double(z1) : nanv;
@@ -344,44 +350,42 @@ __device__ void ldlt_solve_blocked(const T* H, int n, int ldH, const T* dinv, X*
 
 // x = A^-1 b (or -A^-1 b with neg) by the calling warp alone (all 32 lanes;
 // no block barrier) with the LDL^T that ldlt_blocked left in H and dinv:
-// lanes own rows lane and lane + 32 (n <= 64); forward z = D^-1 L^-1 b with
-// the pivot broadcast by shuffles, then backward x = L^-T z.  b is read before
-// x is written (they may alias).  `ok` false (a pivot not positive / finite,
-// ldlt_pivots_ok_warp) makes x NaN.
+// lanes own rows lane and lane + 32 (n <= 64).  Forward, y_k / d_k goes round
+// by a shuffle and each later row subtracts W_ik times it; backward as in
+// ldlt_backward_lanes.  b is read before x is written (they may alias).  `ok`
+// false (a pivot not positive / finite, ldlt_pivots_ok_warp) makes x NaN.
+// (35 DOFs, forward and backward, alone on an SM: 8.7 k cycles with the
+// pivots read per row and the owner of a row selected by branches.)
 template <typename T>
-__device__ void ldlt_solve_warp(const T* H, int n, int ldH, const T* dinv, const double* b, double* x,
-                                bool neg, bool ok) {
+__device__ __forceinline__ void ldlt_solve_warp(const T* H, int n, int ldH, const T* dinv, const double* b, double* x,
+                                                bool neg, bool ok) {
   const int lane = threadIdx.x & 31;
   const T sg = neg ? T(-1) : T(1);
+  const T d0 = lane < n ? dinv[lane] : T(1), d1 = lane + 32 < n ? dinv[lane + 32] : T(1);
   T h0 = lane < n ? sg * T(b[lane]) : T(0);
   T h1 = lane + 32 < n ? sg * T(b[lane + 32]) : T(0);
-#pragma unroll 1
-  for (int k = 0; k < n; ++k) {
-    const T zk = __shfl_sync(0xffffffffu, k < 32 ? h0 : h1, k & 31) * dinv[k];
-    if (lane == (k & 31)) {
-      if (k < 32) h0 = zk;
-      else h1 = zk;
-    }
-    if (lane > k && lane < n) h0 -= H[(size_t)lane * ldH + k] * zk;
-    if (lane + 32 > k && lane + 32 < n) h1 -= H[(size_t)(lane + 32) * ldH + k] * zk;
+  const T* H0 = H + lane * ldH;
+  const T* H1 = H + (lane + 32) * ldH;
+  const bool two = n > 32;
+#pragma unroll 4
+  for (int k = 0; k < (two ? 32 : n); ++k) {
+    const T w0 = lane > k && lane < n ? H0[k] : T(0);
+    const T w1 = lane + 32 < n ? H1[k] : T(0);
+    const T yk = __shfl_sync(0xffffffffu, h0 * d0, k);
+    h0 -= w0 * yk;
+    h1 -= w1 * yk;
   }
-  T s0 = T(0), s1 = T(0);
 #pragma unroll 1
-  for (int i = n - 1; i >= 0; --i) {
-    T xi_local = T(0);
-    if (lane == (i & 31)) {
-      xi_local = i < 32 ? h0 - s0 * dinv[i] : h1 - s1 * dinv[i];
-      if (i < 32) h0 = xi_local;
-      else h1 = xi_local;
-    }
-    const T xi = __shfl_sync(0xffffffffu, xi_local, i & 31);
-    if (lane < i) s0 += H[(size_t)i * ldH + lane] * xi;
-    if (lane + 32 < i) s1 += H[(size_t)i * ldH + lane + 32] * xi;
+  for (int k = 32; k < n; ++k) {
+    const T w1 = lane + 32 > k && lane + 32 < n ? H1[k] : T(0);
+    h1 -= w1 * __shfl_sync(0xffffffffu, h1 * d1, k - 32);
   }
+  T z0 = h0 * d0, z1 = h1 * d1;
+  ldlt_backward_lanes(H, n, ldH, d0, d1, z0, z1);
   const double nanv = __longlong_as_double(0x7ff8000000000000ULL);
   __syncwarp();
-  if (lane < n) x[lane] = ok ? double(h0) : nanv;
-  if (lane + 32 < n) x[lane + 32] = ok ? double(h1) : nanv;
+  if (lane < n) x[lane] = ok ? double(z0) : nanv;
+  if (lane + 32 < n) x[lane + 32] = ok ? double(z1) : nanv;
 }
 
 // Whether every pivot of a stored LDL^T is positive and finite (the warp's

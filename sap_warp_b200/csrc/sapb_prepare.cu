@@ -85,7 +85,7 @@ __host__ __device__ inline PrepLayout prep_layout(int B, int n, int C, int tb) {
   }
   L.S = take(sizeof(double) * 6 * n);       // motion subspace columns
   L.F = take(sizeof(double) * 6 * n);       // composite inertia times S
-  L.vec = take(sizeof(double) * 4 * n);     // tau, vdot, diag(A), 1/d
+  L.vec = take(sizeof(double) * 4 * n);     // tau, vdot, 1 / diag(A), 1/d
   // per contact: x0 3, x1 3, frame 9; before the contacts are set up, X_FM
   // of each body's joint (8 per body) lives in the same bytes
   {
@@ -225,8 +225,15 @@ __device__ __forceinline__ void pose_store(double* p, Xf x) {
 // columns (sim/contact_jacobian.py:404-562).
 // VS: the candidate start velocity is written (v_start; a separate
 // instantiation keeps its registers off the plain path).
+//
+// Bound by latency (short phases between barriers) and by the instruction
+// cache: loops over bodies, DOFs and contacts are not unrolled -- they run
+// once or twice a world, and their bodies are hundreds of instructions.
+// CTAs per SM by measurement, 4096 humanoids: without the start velocity 314 /
+// 283 / 294 us at 5 / 6 / 7, with it (eight learned steps) 7.76 / 7.83 / 7.96
+// ms: more worlds in flight against registers spilled and lines evicted.
 template <bool VS>
-__global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepParams P) {
+__global__ void __launch_bounds__(kPrepNT, VS ? 5 : 6) prepare_world_kernel(const PrepParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x;
   const int e = blockIdx.x;
@@ -255,7 +262,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   double* Fi = reinterpret_cast<double*>(smem + L.F);
   double* tau = reinterpret_cast<double*>(smem + L.vec);
   double* vdot = tau + n;
-  double* adiag = tau + 2 * n;
+  double* ainv = tau + 2 * n;
   double* dinv = tau + 3 * n;
   double* H = reinterpret_cast<double*>(smem + L.H);
   double* pan = Fi;  // the factor's scaled panel: 6 a row, once A is formed from F
@@ -278,14 +285,18 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   const double* qd = P.in.joint_qd;
 
   // ---- topology of this world --------------------------------------------
+#pragma unroll 1
   for (int b = tid; b < B; b += kPrepNT) {
     bj[b] = -1;
     if (blk) btree[b] = -1;
   }
+#pragma unroll 1
   for (int i = tid; i < n; i += kPrepNT) dbody[i] = -1;
   if (!blk) build_triangle_list<kPrepNT>(tri, n, 0);
+#pragma unroll 1
   for (int k = tid; k < 6 * n; k += kPrepNT) S[k] = 0.0;
   if (want_vstart)
+#pragma unroll 1
     for (int k = tid; k < (kPrepNT / 32) * n; k += kPrepNT) jg[k] = 0.0;
   // whether a live slot holds a new contact (the factor is then written
   // under factor_new_contacts_only)
@@ -293,12 +304,14 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   if (P.o.factor_new_contacts_only && P.hist_depth) {
     const int tot = P.env_count[e];
     const int c0 = tot < C ? tot : C;
+#pragma unroll 1
     for (int c = tid; c < c0; c += kPrepNT)
       if (P.hist_depth[(size_t)e * C + c] == 0) newc = 1;
   } else {
     newc = 1;
   }
   __syncthreads();
+#pragma unroll 1
   for (int jl = tid; jl < Jw; jl += kPrepNT) {
     const int j = j0 + jl;
     const int cb = P.m.joint_child[j] - b0g;
@@ -311,6 +324,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   }
   // the trees of the tree-blocked outputs: the world's articulations, each a
   // contiguous DOF range
+#pragma unroll 1
   for (int t = tid; t < ntree; t += kPrepNT) {
     const int ja = P.m.articulation_start[ws.a0 + t], jb = P.m.articulation_start[ws.a0 + t + 1];
     tds[t] = P.m.joint_qd_start[ja] - d0;
@@ -328,6 +342,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   bool tree_bad = false;
   if (blk) {
     bool bad = false;
+#pragma unroll 1
     for (int t = tid; t < ntree; t += kPrepNT) {
       const int cnt = tds[t + 1] - tds[t];
       bad = bad || cnt < 0 || cnt > tb || tds[t] < 0 || tds[t + 1] > n;
@@ -337,6 +352,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
 
   // ---- local transforms X_{parent body, body} = X_p X_FM(q) X_c^-1 ---------
   // (sim/sap_helpers.py:1164-1243)
+#pragma unroll 1
   for (int b = tid; b < B; b += kPrepNT) {
     const int j = bj[b];
     Xf T{v3(0, 0, 0), qident()}, X_FM{v3(0, 0, 0), qident()};
@@ -358,8 +374,9 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
         d6_mobilizer(P.m.joint_axis + 3 * (size_t)ds, q + qs, P.m.joint_dof_dim[2 * j], P.m.joint_dof_dim[2 * j + 1],
                      &X_FM, ax);
       }
-      T = xf_compose(xf_compose(xf_load(P.m.joint_X_p + 7 * (size_t)j), X_FM),
-                     xf_inverse(xf_load(P.m.joint_X_c + 7 * (size_t)j)));
+      X_FM = xf_unit(X_FM);
+      T = xf_compose_unit(xf_compose_unit(xf_unit(xf_load(P.m.joint_X_p + 7 * (size_t)j)), X_FM),
+                          xf_inverse(xf_load(P.m.joint_X_c + 7 * (size_t)j)));
       parent = P.m.joint_parent[j] >= 0 ? P.m.joint_parent[j] - b0g : -1;
       if (parent >= B) parent = -1;
     }
@@ -377,12 +394,14 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   int* jn = jmpB;
   uint64_t* ac = ancA;
   uint64_t* an = ancB;
+#pragma unroll 1
   for (int round = 0; round < 8; ++round) {
     int active = 0;
+#pragma unroll 1
     for (int b = tid; b < B; b += kPrepNT) {
       const int J = jc[b];
       if (J >= 0) {
-        pose_store(nxt + 8 * b, xf_compose(pose_load(cur + 8 * J), pose_load(cur + 8 * b)));
+        pose_store(nxt + 8 * b, xf_compose_unit(pose_load(cur + 8 * J), pose_load(cur + 8 * b)));
         jn[b] = jc[J];
         an[b] = ac[b] | ac[J];
         active = 1;
@@ -410,9 +429,11 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   int* deep_order = reinterpret_cast<int*>(an);
 
   // ---- motion subspaces, joint velocities, body inertias ------------------
+#pragma unroll 1
   for (int b = tid; b < B; b += kPrepNT) {
     const int db = __popcll(anc[b]);  // depth + 1
     int rank = 0;
+#pragma unroll 2
     for (int d = 0; d < B; ++d) {
       const int dd = __popcll(anc[d]);
       rank += (dd > db || (dd == db && d < b)) ? 1 : 0;
@@ -424,6 +445,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   // ball [w_k; p_F x w_k], free [w_k; p_M x w_k] and [0; a_k], all axes
   // rotated by R_WF.
   const V3 grav = load3(P.m.gravity + 3 * (size_t)e);
+#pragma unroll 1
   for (int b = tid; b < B; b += kPrepNT) {
     const int j = bj[b];
     Sv vJ = sv_zero(), c = sv_zero();
@@ -432,9 +454,9 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
       const int ds = P.m.joint_qd_start[j], dl = ds - d0;
       const int parent = P.m.joint_parent[j] >= 0 ? P.m.joint_parent[j] - b0g : -1;
       const Xf X_Wl = (parent >= 0 && parent < B) ? pose_load(pose + 8 * parent) : Xf{v3(0, 0, 0), qident()};
-      const Xf X_WF = xf_compose(X_Wl, xf_load(P.m.joint_X_p + 7 * (size_t)j));
-      const Xf X_WM = xf_compose(X_WF, pose_load(fm + 8 * b));
-      const Q4 R = qnormalize(X_WF.q);
+      const Xf X_WF = xf_compose_unit(X_Wl, xf_unit(xf_load(P.m.joint_X_p + 7 * (size_t)j)));
+      const V3 p_WM = X_WF.p + qrot(X_WF.q, pose_load(fm + 8 * b).p);
+      const Q4 R = X_WF.q;
       auto put = [&](int k, Sv s) {
         sv_store(S + 6 * (dl + k), s);
         vJ = vJ + qd[ds + k] * s;
@@ -452,7 +474,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
       } else if (jt == SAPB_JOINT_FREE || jt == SAPB_JOINT_DISTANCE) {
         for (int k = 0; k < 3; ++k) {
           const V3 w = qrot(R, v3(k == 0, k == 1, k == 2));
-          put(k, sv(w, cross(X_WM.p, w)));
+          put(k, sv(w, cross(p_WM, w)));
           put(k + 3, sv(v3(0, 0, 0), w));
         }
         // the DOFs' own motion: d/dt of p_M x w_k along the relative
@@ -476,7 +498,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
         }
         for (int k = 0; k < ang && k < 3; ++k) {
           const V3 w = qrot(R, ax[k]);
-          put(lin + k, sv(w, cross(X_WM.p, w)));
+          put(lin + k, sv(w, cross(p_WM, w)));
           w_rel = w_rel + qd[ds + lin + k] * w;
         }
         c = sv(v3(0, 0, 0), cross(v_rel, w_rel));
@@ -486,7 +508,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     sv_store(cbias + 6 * b, c);
     // inertia about the world origin (sim/sap_helpers.py:1027-1062)
     const Xf X = pose_load(pose + 8 * b);
-    const Q4 qb = qnormalize(X.q);
+    const Q4 qb = X.q;
     const double m = P.m.body_mass[b0g + b];
     const double* Ic = P.m.body_inertia + 9 * (size_t)(b0g + b);
     const V3 cw = X.p + qrot(qb, load3(P.m.body_com + 3 * (size_t)(b0g + b)));
@@ -515,39 +537,10 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     I[9] = IW[1][2] - m * cw.y * cw.z;
   }
   __syncthreads();
-  // ---- body velocities: sums of the ancestors' joint velocities -------------
-  for (int b = tid; b < B; b += kPrepNT) {
-    Sv v = sv_zero();
-    uint64_t mk = anc[b];
-    while (mk) {
-      const int d = __ffsll((long long)mk) - 1;
-      mk &= mk - 1;
-      v = v + sv_load(vj + 6 * d);
-    }
-    sv_store(vb + 6 * b, v);
-  }
-  __syncthreads();
-  // joint bias accelerations c_b = v_parent x vJ_b (+ the free-joint term)
-  for (int b = tid; b < B; b += kPrepNT) {
-    const int j = bj[b];
-    if (j < 0) continue;
-    const int parent = P.m.joint_parent[j] >= 0 ? P.m.joint_parent[j] - b0g : -1;
-    if (parent < 0 || parent >= B) continue;
-    sv_store(cbias + 6 * b, sv_load(cbias + 6 * b) + crm(sv_load(vb + 6 * parent), sv_load(vj + 6 * b)));
-  }
-  __syncthreads();
-  // ---- body forces f = I a + v x* I v - f_gravity + body_f -------------------
-  // (sim/sap_helpers.py:1065-1105; gravity as the base acceleration -g)
-  for (int b = tid; b < B; b += kPrepNT) {
-    Sv a = sv(v3(0, 0, 0), -grav);
-    uint64_t mk = anc[b];
-    while (mk) {
-      const int d = __ffsll((long long)mk) - 1;
-      mk &= mk - 1;
-      a = a + sv_load(cbias + 6 * d);
-    }
+  // body forces f = I a + v x* I v - f_gravity + body_f (sim/sap_helpers.py:
+  // 1065-1105; gravity as the base acceleration -g)
+  auto body_force = [&](int b, Sv a, Sv v) {
     const double* I = ib + 10 * b;
-    const Sv v = sv_load(vb + 6 * b);
     Sv f = inertia_times(I, a) + crf(v, inertia_times(I, v));
     if (P.in.body_f) {
       const Sv bf = sv_load(P.in.body_f + 6 * (size_t)(b0g + b));  // at the body origin
@@ -555,16 +548,84 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
       f = f + Sv{bf.w + cross(pb, bf.v), bf.v};
     }
     sv_store(fb + 6 * b, f);
+  };
+  if (B <= 32) {
+    // one warp, a body a lane: velocities and bias accelerations are sums
+    // over the ancestors, by pointer jumping through shuffles (five rounds
+    // without a barrier; walking the ancestors took up to 30 dependent steps
+    // a sum)
+    if (tid < 32) {
+      const int b = tid, par_b = b < B ? par[b] : -1;
+      auto shfl_sv = [&](Sv v, int src) {
+        return sv(v3(__shfl_sync(~0u, v.w.x, src), __shfl_sync(~0u, v.w.y, src), __shfl_sync(~0u, v.w.z, src)),
+                  v3(__shfl_sync(~0u, v.v.x, src), __shfl_sync(~0u, v.v.y, src), __shfl_sync(~0u, v.v.z, src)));
+      };
+      auto up_sum = [&](Sv v) {
+        int jump = par_b;
+#pragma unroll 1
+        while (__any_sync(~0u, jump >= 0)) {
+          const int src = jump >= 0 ? jump : b;
+          const Sv t = shfl_sv(v, src);
+          const int next = __shfl_sync(~0u, jump, src);
+          if (jump >= 0) {
+            v = v + t;
+            jump = next;
+          }
+        }
+        return v;
+      };
+      const Sv vJ = b < B ? sv_load(vj + 6 * b) : sv_zero();
+      const Sv v = up_sum(vJ);
+      const Sv vp = shfl_sv(v, par_b >= 0 ? par_b : b);
+      Sv c = b < B ? sv_load(cbias + 6 * b) : sv_zero();
+      if (par_b >= 0) c = c + crm(vp, vJ);  // c_b = v_parent x vJ_b (+ the free-joint term)
+      const Sv a = sv(v3(0, 0, 0), -grav) + up_sum(c);
+      if (b < B) body_force(b, a, v);
+    }
+  } else {
+    // ---- body velocities: sums of the ancestors' joint velocities
+#pragma unroll 1
+    for (int b = tid; b < B; b += kPrepNT) {
+      Sv v = sv_zero();
+      uint64_t mk = anc[b];
+      while (mk) {
+        const int d = __ffsll((long long)mk) - 1;
+        mk &= mk - 1;
+        v = v + sv_load(vj + 6 * d);
+      }
+      sv_store(vb + 6 * b, v);
+    }
+    __syncthreads();
+    // joint bias accelerations c_b = v_parent x vJ_b (+ the free-joint term)
+#pragma unroll 1
+    for (int b = tid; b < B; b += kPrepNT)
+      if (par[b] >= 0)
+        sv_store(cbias + 6 * b, sv_load(cbias + 6 * b) + crm(sv_load(vb + 6 * par[b]), sv_load(vj + 6 * b)));
+    __syncthreads();
+#pragma unroll 1
+    for (int b = tid; b < B; b += kPrepNT) {
+      Sv a = sv(v3(0, 0, 0), -grav);
+      uint64_t mk = anc[b];
+      while (mk) {
+        const int d = __ffsll((long long)mk) - 1;
+        mk &= mk - 1;
+        a = a + sv_load(cbias + 6 * d);
+      }
+      body_force(b, a, sv_load(vb + 6 * b));
+    }
   }
   __syncthreads();
   // ---- subtree forces and composite inertias: own values, then one pass
   // from the deepest bodies up, each adding its subtree into its parent
+#pragma unroll 1
   for (int k = tid; k < 16 * B; k += kPrepNT) {
     const int b = k >> 4, comp = k & 15;
     fs[k] = comp < 6 ? fb[6 * b + comp] : ib[10 * b + comp - 6];
   }
   __syncthreads();
+#pragma unroll 1
   for (int comp = tid; comp < 16; comp += kPrepNT) {
+#pragma unroll 1
     for (int idx = 0; idx < B; ++idx) {
       const int b = deep_order[idx];
       const int p = par[b];
@@ -573,6 +634,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   }
   __syncthreads();
   // ---- tau = joint_f - S^T f_subtree, F_i = I^c S_i (sim/sap_helpers.py:2090-2118)
+#pragma unroll 1
   for (int i = tid; i < n; i += kPrepNT) {
     const int b = dbody[i];
     Sv F = sv_zero();
@@ -592,6 +654,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     // the padding of a tree with fewer DOFs
     const int bb = tb * tb;
     double* Tm = P.out.tree_mass + (size_t)e * ntree * bb;
+#pragma unroll 1
     for (int k = tid; k < ntree * bb; k += kPrepNT) {
       const int t = k / bb, a = (k - t * bb) / tb, b = k % tb;
       const int s0 = tds[t], nt = tds[t + 1] - s0;
@@ -606,7 +669,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
         }
         if (a == b) {
           v += P.m.joint_armature[d0 + i];
-          adiag[i] = v;
+          ainv[i] = 1.0 / (v < 1.0e-12 ? 1.0e-12 : v);
         }
       }
       H[k] = v;
@@ -614,9 +677,12 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     }
   }
   double* Ag = blk ? nullptr : P.out.dynamics_matrix + (size_t)e * n_slot * n_slot;  // compact, stride n
-  for (int k = tid; k < (blk ? 0 : n * n); k += kPrepNT) {
-    const int i = k / n, j = k - i * n;
-    if (j > i) continue;
+  // (the factorization's triangle list, then the first column)
+  const int below = n * (n - 1) / 2;
+#pragma unroll 1
+  for (int k = tid; k < (blk ? 0 : below + n); k += kPrepNT) {
+    const int ij = k < below ? tri[k] : (k - below) << 8;
+    const int i = ij >> 8, j = ij & 255;
     const int bi = dbody[i], bjj = dbody[j];
     double v = 0.0;
     if (bi >= 0 && bjj >= 0) {
@@ -625,7 +691,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     }
     if (i == j) {
       v += P.m.joint_armature[d0 + i];
-      adiag[i] = v;
+      ainv[i] = 1.0 / (v < 1.0e-12 ? 1.0e-12 : v);
     }
     H[(size_t)i * n + j] = v;
     Ag[(size_t)i * n + j] = v;
@@ -637,6 +703,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   if (blk) {
     // a thread per tree: LDL^T of its block (its own DOFs; H_ab = L_ab d_b
     // below the diagonal, d on it) in place and the solve of its DOFs
+#pragma unroll 1
     for (int t = tid; t < ntree; t += kPrepNT) {
       if (tree_bad) break;
       const int s0 = tds[t], nt = tds[t + 1] - s0;
@@ -669,6 +736,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   ldlt_blocked<kPrepNT, double, 5, 0, 0>(H, n, n, dinv, pan, tri);  // width 5: measured fastest for 35 DOFs
   if (write_factor) {
     double* Lg = P.out.dynamics_factor + (size_t)e * n_slot * n_slot;
+#pragma unroll 1
     for (int k = tid; k < n * n; k += kPrepNT) {
       const int i = k / n, j = k - i * n;
       if (j <= i) Lg[k] = H[k];
@@ -681,6 +749,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   // a named barrier of their own; otherwise the whole block solves first.
   const bool split = !blk && n <= 64;
   if (!blk && !split) {
+#pragma unroll 1
     for (int i = tid; i < n; i += kPrepNT) vdot[i] = tau[i];
     __syncthreads();
     ldlt_solve_blocked<kPrepNT, double>(H, n, n, dinv, vdot, false);
@@ -689,7 +758,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   const int total = P.env_count[e];
   const int cc = total < C ? total : C;
   auto POSE_P = [&](int b) { return v3(pose[8 * b], pose[8 * b + 1], pose[8 * b + 2]); };
-  auto POSE_Q = [&](int b) { return qnormalize(Q4{pose[8 * b + 3], pose[8 * b + 4], pose[8 * b + 5], pose[8 * b + 6]}); };
+  auto POSE_Q = [&](int b) { return Q4{pose[8 * b + 3], pose[8 * b + 4], pose[8 * b + 5], pose[8 * b + 6]}; };  // unit
   if (split && tid < 32) {
     ldlt_solve_warp<double>(H, n, n, dinv, tau, vdot, false, ldlt_pivots_ok_warp<double>(H, n, n));
   } else {
@@ -706,18 +775,23 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   // slots follow the flat buffer's order on every step.
   if (!P.ranked) {  // (the contact history ranks them when it runs first)
     int* tmp = conint;  // 2*C ints, free until the rows below use them
+#pragma unroll 1
     for (int c = wt; c < cc; c += wn) tmp[c] = P.env_src[(size_t)e * C + c];
     wsync();
+#pragma unroll 1
     for (int c = wt; c < cc; c += wn) {
       const int v = tmp[c];
       int rank = 0;
+#pragma unroll 2
       for (int j = 0; j < cc; ++j) rank += tmp[j] < v ? 1 : 0;
       P.env_src[(size_t)e * C + rank] = v;
     }
     wsync();
   }
   if (P.out.contact_source)
+#pragma unroll 1
     for (int c = wt; c < C; c += wn) P.out.contact_source[(size_t)e * C + c] = c < cc ? P.env_src[(size_t)e * C + c] : -1;
+#pragma unroll 1
   for (int c = wt; c < cc; c += wn) {
     const int src = P.env_src[(size_t)e * C + c];
     const int sh0 = P.in.contact_shape0[src], sh1 = P.in.contact_shape1[src];
@@ -770,6 +844,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   }
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = tid; i < n; i += kPrepNT) {
     const double vd = vdot[i];
     P.out.v_star[vs0 + i] = tree_bad ? __longlong_as_double(0x7ff8000000000000ll)
@@ -778,6 +853,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     if (P.out.qd_slots) P.out.qd_slots[vs0 + i] = P.in.joint_qd[d0 + i];
   }
   if (P.out.body_q) {
+#pragma unroll 1
     for (int k = tid; k < 7 * B; k += kPrepNT) {
       const int b = k / 7, c = k - 7 * b;
       P.out.body_q[7 * (size_t)(b0g + b) + c] = pose[8 * b + c];
@@ -799,6 +875,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     // registers, columns lane and lane + 32, up to 64 DOFs; in shared memory beyond
     double jgr0 = 0.0, jgr1 = 0.0;
     const double h = P.in.dt[e];
+#pragma unroll 1
     for (int c = warp; c < cc; c += kPrepNT / 32) {
       const double* cs = con + kConStride * (size_t)c;
       const int lb0 = conint[2 * c], lb1 = conint[2 * c + 1];
@@ -818,7 +895,16 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
         }
       }
       double wq[6] = {0, 0, 0, 0, 0, 0}, vq[3] = {0, 0, 0};
-      const double* gst = want_vstart ? P.gamma_start + 3 * ((size_t)e * C + c) : nullptr;
+      double gam[3] = {0.0, 0.0, 0.0};
+      if (want_vstart) {
+        const double* gst = P.gamma_start + 3 * ((size_t)e * C + c);
+        for (int k = 0; k < 3; ++k) gam[k] = __ldg(gst + k);
+      }
+      const uint64_t on0 = lb0 >= 0 ? anc[lb0] : 0ull, on1 = lb1 >= 0 ? anc[lb1] : 0ull;
+      const V3 x0 = load3(cs), x1 = load3(cs + 3);
+      const V3 f0 = load3(cs + kConFrame), f1 = load3(cs + kConFrame + 3), f2 = load3(cs + kConFrame + 6);
+      double* Jc = Jout + (size_t)c * 3 * ncols;
+#pragma unroll 1
       for (int col = lane; col < ncols; col += 32) {
         V3 rel = v3(0, 0, 0);
         int dof = col;
@@ -829,17 +915,15 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
         const int bcol = dof >= 0 ? dbody[dof] : -1;
         if (bcol >= 0) {
           const Sv sc = sv_load(S + 6 * dof);
-          if (lb1 >= 0 && ((anc[lb1] >> bcol) & 1ull)) rel = rel + (sc.v + cross(sc.w, load3(cs + 3)));
-          if (lb0 >= 0 && ((anc[lb0] >> bcol) & 1ull)) rel = rel - (sc.v + cross(sc.w, load3(cs + 0)));
+          if ((on1 >> bcol) & 1ull) rel = rel + (sc.v + cross(sc.w, x1));
+          if ((on0 >> bcol) & 1ull) rel = rel - (sc.v + cross(sc.w, x0));
         }
-        double rw[3];
-        for (int r = 0; r < 3; ++r) {
-          rw[r] = dot(load3(cs + kConFrame + 3 * r), rel);
-          Jout[((size_t)c * 3 + r) * ncols + col] = rw[r];
-        }
+        const double rw[3] = {dot(f0, rel), dot(f1, rel), dot(f2, rel)};
+#pragma unroll
+        for (int r = 0; r < 3; ++r) Jc[r * ncols + col] = rw[r];
         if (dof < 0) continue;
         if (want_vstart) {
-          const double t = rw[0] * __ldg(gst) + rw[1] * __ldg(gst + 1) + rw[2] * __ldg(gst + 2);
+          const double t = rw[0] * gam[0] + rw[1] * gam[1] + rw[2] * gam[2];
           if (n <= 64) {
             if (col < 32) jgr0 += t;
             else jgr1 += t;
@@ -847,41 +931,38 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
             jg[warp * n + dof] += t;
           }
         }
-        const double vs = P.in.joint_qd[d0 + dof] + h * vdot[dof];
-        vq[0] += rw[0] * vs;
-        vq[1] += rw[1] * vs;
-        vq[2] += rw[2] * vs;
+        if (P.out.vc_star) {
+          const double vs = P.in.joint_qd[d0 + dof] + h * vdot[dof];
+          vq[0] += rw[0] * vs;
+          vq[1] += rw[1] * vs;
+          vq[2] += rw[2] * vs;
+        }
         if (dd) {
-          double aii = adiag[dof];
-          if (aii < 1.0e-12) aii = 1.0e-12;
-          const double inv = 1.0 / aii;
-          wq[0] += inv * rw[0] * rw[0];
-          wq[1] += inv * rw[0] * rw[1];
-          wq[2] += inv * rw[0] * rw[2];
-          wq[3] += inv * rw[1] * rw[1];
-          wq[4] += inv * rw[1] * rw[2];
+          const double inv = ainv[dof];
+          const double i0 = inv * rw[0], i1 = inv * rw[1];
+          wq[0] += i0 * rw[0];
+          wq[1] += i0 * rw[1];
+          wq[2] += i0 * rw[2];
+          wq[3] += i1 * rw[1];
+          wq[4] += i1 * rw[2];
           wq[5] += inv * rw[2] * rw[2];
         }
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) vq[k] += __shfl_xor_sync(0xffffffffu, vq[k], o);
-        if (dd) {
-#pragma unroll
-          for (int k = 0; k < 6; ++k) wq[k] += __shfl_xor_sync(0xffffffffu, wq[k], o);
-        }
+      const size_t ci = (size_t)e * C + c;
+      if (P.out.vc_star) {
+        const double v = warp_sum4(vq[0], vq[1], vq[2], 0.0);
+        if ((lane & 7) == 0 && lane < 24) P.out.vc_star[3 * ci + (lane >> 3)] = v;
       }
-      if (lane == 0) {
-        const size_t ci = (size_t)e * C + c;
-        if (P.out.vc_star)
-          for (int k = 0; k < 3; ++k) P.out.vc_star[3 * ci + k] = vq[k];
-        if (dd) {
-          // ||J diag(A)^-1 J^T||_F / 3 (sim/contact_jacobian.py:153-251)
-          const double wv = sqrt(wq[0] * wq[0] + wq[3] * wq[3] + wq[5] * wq[5] +
-                                 2.0 * (wq[1] * wq[1] + wq[2] * wq[2] + wq[4] * wq[4])) / 3.0;
-          P.out.w_eff[ci] = wv < 1.0e-12 ? 1.0e-12 : wv;
-        }
+      if (dd) {
+        // ||J diag(A)^-1 J^T||_F / 3 (sim/contact_jacobian.py:153-251): the
+        // lanes' sums squared, the off-diagonal ones twice, then over the
+        // four groups of lanes
+        const double sa = warp_sum4(wq[0], wq[3], wq[5], wq[1]), sb = warp_sum4(wq[2], wq[4], 0.0, 0.0);
+        double q = (lane >= 24 ? 2.0 : 1.0) * sa * sa + 2.0 * sb * sb;
+        q += __shfl_xor_sync(0xffffffffu, q, 8);
+        q += __shfl_xor_sync(0xffffffffu, q, 16);
+        const double wv = sqrt(q) / 3.0;
+        if (lane == 0) P.out.w_eff[ci] = wv < 1.0e-12 ? 1.0e-12 : wv;
       }
     }
     if (want_vstart && n <= 64) {
@@ -892,6 +973,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
   __syncthreads();
   // ---- body_inertia contact weights (sim/contact_jacobian.py:153-251) --------
   if (P.o.contact_weight_mode != SAPB_WEIGHT_DIAG_DELASSUS) {
+#pragma unroll 1
   for (int c = tid; c < cc; c += kPrepNT) {
     const size_t ci = (size_t)e * C + c;
     double w = 0.0;
@@ -943,6 +1025,7 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     }
   } else if (want_vstart) {
     __syncthreads();
+#pragma unroll 1
     for (int i = tid; i < n; i += kPrepNT) {
       double r = 0.0;
       for (int q = 0; q < kPrepNT / 32; ++q) r += jg[q * n + i];
@@ -951,11 +1034,13 @@ __global__ void __launch_bounds__(kPrepNT, 7) prepare_world_kernel(const PrepPar
     __syncthreads();
     double* z = jg + n;
     {
+#pragma unroll 1
       for (int i = tid; i < n; i += kPrepNT) z[i] = jg[i];
       __syncthreads();
       ldlt_solve_blocked<kPrepNT, double>(H, n, n, dinv, z, false);
     }
     __syncthreads();
+#pragma unroll 1
     for (int i = tid; i < n; i += kPrepNT)
       P.out.v_start[vs0 + i] = P.in.joint_qd[d0 + i] + P.in.dt[e] * vdot[i] + z[i];
   }
