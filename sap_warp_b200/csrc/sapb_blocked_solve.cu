@@ -44,9 +44,17 @@ int32_t blocked_solve_launch(const sapb_blocked_problem* p, const sapb_solve_opt
   }
   // threads per world: as asked, else 128 for worlds of up to 128 padded
   // DOFs (a few small trees: more worlds in flight between block barriers)
-  // and 256 beyond
+  // and 256 beyond; 512 for free bodies from 360 DOFs on, where one world
+  // fills an SM's shared memory, its warps are all that hides latency and the
+  // block solves' scratch holds the reductions' (296 worlds of 64 boxes, 256
+  // and 512 threads: FP32 armijo_decay 6462 and 6050 us, exact_root 5385 and
+  // 5230; FP64 7820 and 7394, 6741 and 6633; of 54 boxes FP32 exact_root 5089
+  // and 5175)
   int threads = o->threads_per_cta;
-  if (threads != 128 && threads != 256) threads = p->trees_per_env * p->tree_dofs <= 128 ? 128 : 256;
+  if (threads != 128 && threads != 256) {
+    const int n = p->trees_per_env * p->tree_dofs;
+    threads = n <= 128 ? 128 : (p->tree_dofs == 6 && n >= 360 ? 512 : 256);
+  }
   cudaError_t err;
   switch (p->tree_dofs) {
     case 6:

@@ -40,6 +40,7 @@
 
 #include "sapb_device.cuh"
 #include "sapb_internal.h"
+#include "sapb_ldlt.cuh"
 #include "sapb_linesearch.cuh"
 
 namespace sapb {
@@ -540,8 +541,8 @@ __device__ void bfactor(const BWorld<NT, HT, NB>& w) {
 #pragma unroll
         for (int e = 0; e < b; ++e) d -= Lr[b][e] * Lr[b][e] * Dr[e];
         Dr[b] = d;
-        Rr[b] = fast_recip(d);
-        ok = ok && d > HT(0) && isfinite(double(d));
+        Rr[b] = pivot_recip(d);
+        ok = ok && Rr[b] > HT(0) && Rr[b] < HT(INFINITY);  // d positive and finite
 #pragma unroll
         for (int a = b + 1; a < NB; ++a) {
           HT v = Lr[a][b];
@@ -792,7 +793,10 @@ __device__ bool bsymbolic(const BWorld<NT, HT, NB>& w, int cap) {
 template <int NT, typename HT, int NB, int LSV>
 __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double red[2 * kRedBatch * (NT / 32)];
+  // the reductions' scratch; with 512 threads in the place of the block solves'
+  // (not in use beside them), where the static arrays leave no room
+  constexpr int kRed = 2 * kRedBatch * (NT / 32);
+  __shared__ double red_own[NT < 512 ? kRed : 1];
   __shared__ int s_next;
   __shared__ int16_t s_tstart[kBMaxTrees], s_tcount[kBMaxTrees];  // world DOFs: at most 64 x 12
   __shared__ int s_bad_layout;
@@ -849,7 +853,7 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
     w.vec = reinterpret_cast<double*>(smem + L.off_vec);
     w.con = reinterpret_cast<double*>(smem + L.off_con);
     w.flags = reinterpret_cast<int*>(smem + L.off_flags);
-    w.red = red;
+    w.red = NT < 512 ? red_own : reinterpret_cast<double*>(smem + L.off_zd);
     w.A = P.p.tree_mass + (size_t)e * T * NB * NB;
     w.J = P.p.jacobian + (size_t)e * C * 3 * 2 * NB;
     w.tree = reinterpret_cast<const int8_t*>(smem + L.off_tree);
@@ -1271,12 +1275,15 @@ cudaError_t launch_blocked_nt(const BlockedParams& P, cudaStream_t stream) {
 }
 
 // One block size's kernels (both Hessian precisions, 128 or 256 threads per
-// world, every line search), instantiated in a translation unit of its own
+// world, also 512 for free bodies, every line search), instantiated in a translation unit of its own
 // (sapb_blocked_nb{6,7,12}.cu) so they compile in parallel.
 template <int NB>
 cudaError_t launch_blocked(const BlockedParams& P, bool fp32, int threads, cudaStream_t stream) {
   if (threads == 128)
     return fp32 ? launch_blocked_nt<128, float, NB>(P, stream) : launch_blocked_nt<128, double, NB>(P, stream);
+  if constexpr (NB == 6)
+    if (threads == 512)
+      return fp32 ? launch_blocked_nt<512, float, NB>(P, stream) : launch_blocked_nt<512, double, NB>(P, stream);
   return fp32 ? launch_blocked_nt<256, float, NB>(P, stream) : launch_blocked_nt<256, double, NB>(P, stream);
 }
 extern template cudaError_t launch_blocked<6>(const BlockedParams&, bool, int, cudaStream_t);
