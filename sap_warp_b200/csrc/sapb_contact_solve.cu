@@ -52,6 +52,15 @@ int ldlt_block_widths(int n, int32_t* out, int capacity) {
   }
 }
 
+// Whether two worlds of this size do not fit an SM, but one with eight warps does.
+static bool one_per_sm(const sapb_contact_problem& p, bool fp32) {
+  const int hsize = fp32 ? 4 : 8;
+  const size_t per_cta = 1024 + 512;  // reserved per CTA, and the kernel's static arrays
+  return !p.dof_count && !specialised_dofs(p.dof_per_env) &&
+         2 * (make_layout(p.dof_per_env, p.max_contacts, hsize, 128).total + per_cta) > 228 * 1024 &&
+         make_layout(p.dof_per_env, p.max_contacts, hsize, 256).total <= kMaxSmemPerBlock;
+}
+
 static cudaError_t solve_sized(const SolveParams& P, int n, bool fp32, cudaStream_t stream, int* blocks_out) {
   switch (n) {
 #define SAPB_DISPATCH_N(NV) \
@@ -70,8 +79,11 @@ static cudaError_t solve_sized(const SolveParams& P, int n, bool fp32, cudaStrea
 static cudaError_t solve_dispatch(const SolveParams& P, bool fp32, cudaStream_t stream, int* blocks_out) {
   // Kernels specialised on the DOF count of the common trees (humanoid 35,
   // quadruped 18, arm + box 13, single free body 6); a generic one otherwise;
-  // the generic one with eight warps per world on request.
-  if (P.o.threads_per_cta == 256)
+  // the generic one with eight warps per world on request, and by itself for
+  // worlds whose shared memory leaves one CTA per SM, where four warps would
+  // be all that hides latency (512 arm-and-box worlds of 55 DOFs and 112
+  // contact slots, FP64, two steps: 9265 us with 128 threads, 6527 with 256).
+  if (P.o.threads_per_cta == 256 || (P.o.threads_per_cta == 0 && one_per_sm(P.p, fp32)))
     return fp32 ? launch_solve_wide<true>(P, stream, blocks_out) : launch_solve_wide<false>(P, stream, blocks_out);
   if (!P.p.dof_count) return solve_sized(P, P.p.dof_per_env, fp32, stream, blocks_out);
   // Per-world DOF counts: one launch per size class, each kernel taking the
