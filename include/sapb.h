@@ -110,12 +110,13 @@ typedef struct sapb_solve_options {
   int32_t skip_plain_start;       /* nonzero, with candidate starts: start from the best candidate without
                                    * evaluating the plain start (v_guess or v0), which is kept only as the
                                    * fallback when no candidate's cost is finite; 0: the plain start competes */
-  int32_t threads_per_cta;        /* threads of one world's CTA in the dense solve: 0 or 128 the default (the
-                                   * kernel specialised on the DOF count), 256 the runtime-size kernel with
-                                   * eight warps per world (for worlds whose shared memory leaves one or two
-                                   * CTAs per SM); in the tree-blocked solve 128 or 256, 0 picking 128 for
-                                   * worlds of up to 128 padded DOFs (T * tree_dofs) and 256 beyond; results
-                                   * do not depend on it beyond rounding */
+  int32_t threads_per_cta;        /* threads of one world's CTA in the dense solve: 128 (the kernel specialised
+                                   * on the DOF count) or 256 (the runtime-size kernel with eight warps per
+                                   * world), 0 picking 256 where the shared memory of a DOF count without a
+                                   * specialised kernel leaves one CTA per SM and 128 else; in the tree-blocked
+                                   * solve 128 or 256, 0 picking 128 for worlds of up to 128 padded DOFs
+                                   * (T * tree_dofs), 512 for free bodies (tree_dofs 6) from 360 on and 256
+                                   * else; results do not depend on it beyond rounding */
 } sapb_solve_options;
 
 /* Per-DOF drive and limit model (the arrays SapContactSolve.prepare reads,

@@ -3,7 +3,8 @@ around the 8 x 8 Hessian blocks, the factorization's column blocks and the
 32 lanes of its backward substitution, the specialised counts and their
 neighbours, contact counts around the four-row steps; and large uneven
 batches, which run one launch per size class, against the same worlds in
-small ones, which run in one.
+small ones, which run in one; and worlds that fill an SM's shared memory,
+which run eight warps by default.
 
 Tolerances as in test_gpu_contact_solve (same iterates as the oracle up to
 rounding); between the two launches of an uneven batch the worlds run the
@@ -48,6 +49,16 @@ def test_dof_counts_match_oracle(cuda_device, oracle, n, variant):
     ref = oracle.solve(prob, variant)
     assert_parity(prob, gpu, ref)
     np.testing.assert_array_equal(gpu["converged"], ref["converged"])
+
+
+@pytest.mark.parametrize("n, contacts", [(41, 96), (55, 112)])
+def test_worlds_that_fill_an_sm_match_oracle(cuda_device, oracle, n, contacts):
+    prob = scenes.humanoid_contact_problem(6, seed=400 + n, revolute=n - 6, contacts=(contacts // 2, contacts),
+                                           max_contacts=contacts)
+    gpu = run_gpu(prob, cuda_device, "armijo_decay")
+    assert_parity(prob, gpu, oracle.solve(prob, "armijo_decay"))
+    four = run_gpu(prob, cuda_device, "armijo_decay", threads_per_cta=128)
+    assert_parity(prob, gpu, four)
 
 
 def _uneven(worlds: int, dofs, device):
