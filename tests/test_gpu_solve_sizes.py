@@ -4,7 +4,9 @@ around the 8 x 8 Hessian blocks, the factorization's column blocks and the
 neighbours, contact counts around the four-row steps; and large uneven
 batches, which run one launch per size class, against the same worlds in
 small ones, which run in one; and worlds that fill an SM's shared memory,
-which run eight warps by default.
+which run eight warps by default; and free-box worlds around the 360 DOFs
+from which the tree-blocked solve runs 512 threads, against 256 (two answers
+that may take different paths, as in test_gpu_blocked's full-size worlds).
 
 Tolerances as in test_gpu_contact_solve (same iterates as the oracle up to
 rounding); between the two launches of an uneven batch the worlds run the
@@ -19,6 +21,7 @@ import torch
 
 from sap_warp_b200 import scenes
 from sap_warp_b200._solve import ContactSolveBuffers, contact_solve, make_options, problem_to_device
+from tests.test_gpu_blocked import run_blocked
 from tests.test_gpu_contact_solve import assert_parity, run_gpu
 
 pytestmark = pytest.mark.gpu
@@ -59,6 +62,17 @@ def test_worlds_that_fill_an_sm_match_oracle(cuda_device, oracle, n, contacts):
     assert_parity(prob, gpu, oracle.solve(prob, "armijo_decay"))
     four = run_gpu(prob, cuda_device, "armijo_decay", threads_per_cta=128)
     assert_parity(prob, gpu, four)
+
+
+@pytest.mark.parametrize("boxes", [59, 60, 63])
+@pytest.mark.parametrize("variant", ["armijo_decay", "exact_root"])
+def test_wide_box_worlds_match_256_threads(cuda_device, boxes, variant):
+    bp = scenes.box_stack_problem(4, seed=460 + boxes, boxes=boxes)
+    gpu = run_blocked(bp, cuda_device, variant)
+    narrow = run_blocked(bp, cuda_device, variant, threads_per_cta=256)
+    np.testing.assert_array_equal(gpu["converged"], narrow["converged"])
+    np.testing.assert_array_equal(gpu["status"], 0)
+    assert_parity(bp.to_dense(), gpu, narrow, max_loose_frac=0.5)
 
 
 def _uneven(worlds: int, dofs, device):
