@@ -234,7 +234,9 @@ typedef struct sapb_solve_outputs {
  * joints, bodies, DOFs and coordinates (the layout the reference requires,
  * sim/contact_solve.py:3327-3335).  Arrays are global (all worlds), indices
  * global, as in SapModel (sim/sap_runtime.py:47-174).  Joints are ordered
- * parents before children within each articulation. */
+ * parents before children within each articulation; no body is among its own
+ * ancestors (the arrays are on the device and not checked for it: such a world
+ * has no defined result). */
 typedef struct sapb_model_desc {
   int32_t num_worlds;
   int32_t joints_per_world;

@@ -551,9 +551,9 @@ __global__ void __launch_bounds__(kPrepNT, VS ? 5 : 6) prepare_world_kernel(cons
   };
   if (B <= 32) {
     // one warp, a body a lane: velocities and bias accelerations are sums
-    // over the ancestors, by pointer jumping through shuffles (five rounds
-    // without a barrier; walking the ancestors took up to 30 dependent steps
-    // a sum)
+    // over the ancestors, by pointer jumping through shuffles (at most five
+    // rounds, which reach 31 ancestors, whatever the parents hold; no barrier;
+    // walking the ancestors took up to 30 dependent steps a sum)
     if (tid < 32) {
       const int b = tid, par_b = b < B ? par[b] : -1;
       auto shfl_sv = [&](Sv v, int src) {
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(kPrepNT, VS ? 5 : 6) prepare_world_kernel(cons
       auto up_sum = [&](Sv v) {
         int jump = par_b;
 #pragma unroll 1
-        while (__any_sync(~0u, jump >= 0)) {
+        for (int round = 0; round < 5 && __any_sync(~0u, jump >= 0); ++round) {
           const int src = jump >= 0 ? jump : b;
           const Sv t = shfl_sv(v, src);
           const int next = __shfl_sync(~0u, jump, src);

@@ -122,6 +122,7 @@ class _ModelView:
         parent_joint = model.joint_ancestor.cpu().numpy()
         if np.any(parent_joint >= np.arange(J)):
             raise ValueError("joints must be ordered parents before children")
+        self._check_body_tree()
         self.device = model.joint_type.device
         # the tree-blocked layout: the trees are the world's articulations
         # (a free body, an arm), each in a block of tree_block DOFs (6, 7 or
@@ -175,6 +176,35 @@ class _ModelView:
             self.dof_count_t = None
         self.desc = d
         self._build_dof_maps(jt)
+
+    def _check_body_tree(self):
+        """Refuse a model with a body among its own ancestors.  As in the free
+        motion, a joint links two bodies of its own world (a parent outside it
+        is the ground)."""
+        m = self.model
+        J, B = int(m.joint_count), int(m.body_count)
+        parent = m.joint_parent.cpu().numpy().astype(np.int64)[:J]
+        child = m.joint_child.cpu().numpy().astype(np.int64)[:J]
+        live = (parent >= 0) & (parent < B) & (child >= 0) & (child < B)
+        joint, parent, child = np.flatnonzero(live), parent[live], child[live]
+        if self.uneven:
+            jworld = np.searchsorted(self.world_offsets["joint"], joint, side="right")
+            pworld, cworld = (np.searchsorted(self.world_offsets["body"], b, side="right") for b in (parent, child))
+        else:
+            jworld, pworld, cworld = joint // self.Jw, parent // self.Bw, child // self.Bw
+        own = (pworld == cworld) & (jworld == cworld)
+        parent, child = parent[own], child[own]
+        # from the roots down, a level a pass: a body hangs while its parent does
+        hangs = np.ones(B, bool)
+        while True:
+            below = np.zeros(B, bool)
+            below[child[hangs[parent]]] = True
+            if np.array_equal(below, hangs):
+                break
+            hangs = below
+        if hangs.any():
+            raise ValueError(f"joint_parent holds a cycle: body {int(np.flatnonzero(hangs)[0])} is among its own "
+                             "ancestors or below such a body")
 
     def _build_dof_maps(self, jt):
         """sim/contact_solve.py:3681-3758: DOF -> coordinate, drive target and
