@@ -222,23 +222,38 @@ __device__ __forceinline__ double sum_partials(const World<NT, HT, NS>& w, int w
 
 enum EvalStart { kEvalFull = 0, kEvalStep = 1, kEvalSame = 2 };
 
+// vc and a_res, moved along line searches since they were formed, have to be
+// formed again when v or v - v* has become small against what they went
+// through.  Formed, their rounding errors are of the order of eps times
+// |J| |v| and |A| |v - v*|; moved, they keep those of the largest v and v - v*
+// on the way, and each step adds its own.  So the square of the largest size
+// (in the norm of diag(A)) grows by half a step, and at sixteen times the
+// present one -- a fourth of the size, or seven steps -- they are formed
+// again: a start of the solution's size rarely gets there, one far from it (a
+// poor guess or candidate) does so on its way in.  (From a guess 1e8 times too
+// large the gradient at the returned velocity was 1e4 times the tolerance it
+// was reported to meet when they were never formed again.)
+constexpr double kSeenGrowth = 1.5, kSeenLimit = 16.0;
+
 // Objective at the current v: contact impulses, costs and derivatives G,
 // a_res = A(v - v*), J^T gamma, PD and limit terms, gradient (and its negative
 // as the factorization's right-hand-side row).  Returns {cost, |g|^2, |p|^2,
-// |jc|^2} (scaled, over participating DOFs) and the momentum cost
-// 1/2 (v - v*) a_res to every thread.  Restates _solver_update_active
+// |jc|^2} (scaled, over participating DOFs), the momentum cost
+// 1/2 (v - v*) a_res and whether the moved vc and a_res are too old
+// (kSeenLimit) to every thread.  Restates _solver_update_active
 // sim/contact_solve.py:4080-4136.
 //
 // kEvalFull forms vc = J v and a_res from V_V; kEvalStep moves v, vc and
 // a_res by alpha times dv, J dv and A dv of the line search (all linear in v:
-// a Newton step then reads neither A nor J here but for J^T gamma); kEvalSame
-// leaves them.  The first two warps hold the DOFs; of the others every second
+// a Newton step then reads neither A nor J here but for J^T gamma; kSeenLimit
+// says when they are formed again); kEvalSame leaves them.  The first two warps hold the DOFs; of the others every second
 // one projects the contacts for impulses and costs and the rest for the
 // derivatives, side by side (the projection is a long dependent chain of few
 // threads).
 template <int NT, typename HT, int NS>
 __device__ __forceinline__ void evaluate(const World<NT, HT, NS>& w, const SolveParams& P, double dt, int start,
-                                         bool first, double alpha, double out4[4], double* mom) {
+                                         bool first, double alpha, double out4[4], double* mom,
+                                         bool* too_old) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int NW = NT / 32, kStride = 32 * (NW - 2) / 2;
   const int n = w.dofs();
@@ -358,9 +373,29 @@ __device__ __forceinline__ void evaluate(const World<NT, HT, NS>& w, const Solve
     if ((lane & 7) == 0) r[lane >> 3] = tot;
     if (P.dof.has_pd || P.dof.has_limits) extra = warp_sum<NT>(extra);
     if (lane == 0) r[4] = extra;
+  } else if (warp == 1) {  // the sizes of v and v - v*
+    double sv = 0.0, sr = 0.0;
+#pragma unroll 1
+    for (int i = lane; i < n; i += 32) {
+      const double vi = w.V(V_V)[i], ri = vi - w.V(V_VSTAR)[i], d = w.V(V_ADIAG)[i];
+      sv += d * vi * vi;
+      sr += d * ri * ri;
+    }
+    const double now = warp_sum4(sv, sr, 0.0, 0.0);
+    double* r = w.red + kRedEval * NW;
+    static_assert(8 <= (kRedSize - kRedEval) * NW, "the evaluation's sums");
+    bool old = false;
+    if (lane == 0 || lane == 8) {
+      double* seen = r + 6 + (lane >> 3);
+      const double m = start == kEvalFull ? now : (start == kEvalStep ? fmax(kSeenGrowth * *seen, now) : *seen);
+      *seen = m;
+      old = m > kSeenLimit * now;
+    }
+    old = __any_sync(0xffffffffu, old);
+    if (lane == 0) r[5] = old ? 1.0 : 0.0;
   } else if (start == kEvalStep) {  // the moved contact velocities (their old ones are read)
 #pragma unroll 1
-    for (int q = tid - 32; q < 3 * w.count; q += NT - 32) {
+    for (int q = tid - 64; q < 3 * w.count; q += NT - 64) {
       const int k = q / w.count, c = q - k * w.count;
       w.cn(c)[C_VC + k] += alpha * w.cn(c)[C_DVC + k];
     }
@@ -375,6 +410,7 @@ __device__ __forceinline__ void evaluate(const World<NT, HT, NS>& w, const Solve
   out4[1] = r[1];
   out4[2] = r[2];
   out4[3] = r[3];
+  *too_old = r[5] != 0.0;
 }
 
 // H (lower triangle, HT) <- the lower triangle of the FP64 n x n matrix M in
@@ -686,7 +722,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
         w.V(V_V)[i] = v;
         double d = __ldg(w.A + (size_t)i * n + i);
         if (d < 1.0e-12 || !isfinite(d)) d = 1.0e-12;
-        w.V(V_AINV)[i] = 1.0 / d;
+        w.V(V_ADIAG)[i] = d;
         w.V(V_DSCALE)[i] = 1.0 / sqrt(d);
       } else {
         for (int k = 0; k < kVecs; ++k) w.V(k)[i] = 0.0;
@@ -710,7 +746,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
         const double kp = (double)D.joint_target_ke[target], kd = (double)D.joint_target_kd[target];
         if (!(kp <= 0.0 && kd <= 0.0) && !(coord < 0 && kp > 0.0)) {
           double kpe, kde;
-          effective_pd_gains(kp, kd, dt, w.V(V_AINV)[i], &kpe, &kde);
+          effective_pd_gains(kp, kd, dt, 1.0 / w.V(V_ADIAG)[i], &kpe, &kde);
           const double gain = dt * kpe + kde;
           if (gain > 0.0) {
             double q0 = 0.0, qd = 0.0;
@@ -742,7 +778,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
         const double kd = D.joint_limit_kd[dof];
         const double tau_d = kd > 0.0 ? kd / ke : 0.0;
         const double bf = kLimitBeta * kLimitBeta / (4.0 * kPi * kPi);
-        const double r_nr = bf * fmax(w.V(V_AINV)[i], 1.0e-12);
+        const double r_nr = bf * fmax(1.0 / w.V(V_ADIAG)[i], 1.0e-12);
         const double r_soft = 1.0 / (dt * ke * (dt + tau_d));
         const double rr = fmax(r_nr, r_soft);
         if (isfinite(lower) && q0 - lower <= window) {
@@ -953,8 +989,13 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
         __syncthreads();
       }
       double e4[4], mom;
-      evaluate<NT, HT, NS>(w, P, dt, from, first, alpha, e4, &mom);
+      bool too_old;
+      evaluate<NT, HT, NS>(w, P, dt, from, first, alpha, e4, &mom, &too_old);
       first = false;
+      if (too_old) {
+        from = kEvalFull;
+        continue;
+      }
       if (start >= 0) {
         if (start == 0) {
           best_cost = e4[0];

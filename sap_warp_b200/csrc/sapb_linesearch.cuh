@@ -24,7 +24,8 @@ constexpr int kFlagPd = 1, kFlagLo = 2, kFlagUp = 4, kFlagPart = 8;
 enum Vec {
   V_V = 0, V_VSTAR, V_DV, V_GRAD, V_ARES, V_DP, V_DSCALE, V_AINV, V_PDA, V_PDGAIN, V_PDLIM,
   V_LOVHAT, V_UPVHAT, V_LOR, V_UPR, V_LORINV, V_UPRINV, V_HDIAG, V_TMP0, V_SAVE, V_BEST, V_DINV, V_END,
-  V_AVS = V_TMP0  // the dense solve's A v*
+  V_AVS = V_TMP0,   // the dense solve's A v*
+  V_ADIAG = V_AINV  // the dense solve's diag(A)
 };
 // A contact's record of C_END doubles: one address per contact and constant
 // offsets, and 17 of them (odd) keep a warp's accesses, a contact a lane, free
