@@ -530,26 +530,35 @@ __device__ void bfactor(const BWorld<NT, HT, NB>& w) {
       const int j = w.iw[BI_LNODES + idx];
       HT* Fj = w.F + j * NB * NB;
       HT Lr[NB][NB], Dr[NB], Rr[NB];
+      auto factor_block = [&](auto divide) {
+        bool normal = true;
 #pragma unroll
-      for (int a = 0; a < NB; ++a)
+        for (int a = 0; a < NB; ++a)
 #pragma unroll
-        for (int b = 0; b <= a; ++b) Lr[a][b] = Fj[a * NB + b];
-      bool ok = true;
+          for (int b = 0; b <= a; ++b) Lr[a][b] = Fj[a * NB + b];
 #pragma unroll
-      for (int b = 0; b < NB; ++b) {
-        HT d = Lr[b][b];
+        for (int b = 0; b < NB; ++b) {
+          HT d = Lr[b][b];
 #pragma unroll
-        for (int e = 0; e < b; ++e) d -= Lr[b][e] * Lr[b][e] * Dr[e];
-        Dr[b] = d;
-        Rr[b] = pivot_recip(d);
-        ok = ok && Rr[b] > HT(0) && Rr[b] < HT(INFINITY);  // d positive and finite
+          for (int e = 0; e < b; ++e) d -= Lr[b][e] * Lr[b][e] * Dr[e];
+          Dr[b] = d;
+          Rr[b] = pivot<decltype(divide)::value>(d);
+          normal &= positive_normal(Rr[b]);
 #pragma unroll
-        for (int a = b + 1; a < NB; ++a) {
-          HT v = Lr[a][b];
+          for (int a = b + 1; a < NB; ++a) {
+            HT v = Lr[a][b];
 #pragma unroll
-          for (int e = 0; e < b; ++e) v -= Lr[a][e] * Lr[b][e] * Dr[e];
-          Lr[a][b] = v * Rr[b];
+            for (int e = 0; e < b; ++e) v -= Lr[a][e] * Lr[b][e] * Dr[e];
+            Lr[a][b] = v * Rr[b];
+          }
         }
+        return normal;
+      };
+      bool ok = true;
+      if (__builtin_expect(!factor_block(std::false_type{}), 0)) {
+        factor_block(std::true_type{});
+#pragma unroll
+        for (int b = 0; b < NB; ++b) ok = ok && Dr[b] > HT(0) && isfinite(double(Dr[b]));
       }
 #pragma unroll
       for (int a = 0; a < NB; ++a) {

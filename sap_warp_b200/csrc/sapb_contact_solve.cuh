@@ -117,6 +117,7 @@ struct World {
   int* flags;
   const uint16_t* tri;
   double* red;
+  const double* scale;  // shared: the power of two that H and its right-hand sides carry (WorldScale)
   int* factor_ok;  // shared: whether the last Newton factorization's pivots were all positive and finite
   int n, count;
   // DOF count and leading dimensions: compile-time constants when NS > 0.
@@ -321,6 +322,7 @@ __device__ __forceinline__ void evaluate(const World<NT, HT, NS>& w, const Solve
   if (warp == 0) {  // gradient and norms: two DOFs a lane
     double mterm = 0.0, extra = 0.0, g2 = 0.0, p2 = 0.0, j2 = 0.0;
     HT* rhs = w.H + n * w.ldH();
+    const double scale = *w.scale;
 #pragma unroll 1
     for (int i = lane; i < n; i += 32) {
       double imp = sum_partials<NT, HT, NS>(w, 0, i);
@@ -359,7 +361,7 @@ __device__ __forceinline__ void evaluate(const World<NT, HT, NS>& w, const Solve
       const double grad = a_res - imp;
       w.V(V_GRAD)[i] = grad;
       w.V(V_HDIAG)[i] = hd;
-      rhs[i] = HT(-grad);
+      rhs[i] = HT(-grad * scale);
       if (fl & kFlagPart) {
         const double s = w.V(V_DSCALE)[i];
         const double gs = s * grad, ps = s * a_v, js = s * imp;
@@ -414,13 +416,13 @@ __device__ __forceinline__ void evaluate(const World<NT, HT, NS>& w, const Solve
 }
 
 // H (lower triangle, HT) <- the lower triangle of the FP64 n x n matrix M in
-// global memory (+ diag_add on the diagonal): flat coalesced reads, four
-// loads in flight per thread.
+// global memory, scaled: flat coalesced reads, four loads in flight per thread.
 template <int NT, typename HT, int NS>
 __device__ __forceinline__ void load_lower(const World<NT, HT, NS>& w, const double* M) {
   const int tid = threadIdx.x;
   const int n = w.dofs(), ldH = w.ldH();
   const int total = n * n;
+  const double scale = *w.scale;
 #pragma unroll 1
   for (int k0 = tid; k0 < total; k0 += 4 * NT) {
     double val[4];
@@ -434,7 +436,7 @@ __device__ __forceinline__ void load_lower(const World<NT, HT, NS>& w, const dou
       const int k = k0 + u * NT;
       if (k < total) {
         const int i = k / n, j = k - i * n;
-        if (j <= i) w.H[(size_t)i * ldH + j] = HT(val[u]);
+        if (j <= i) w.H[(size_t)i * ldH + j] = HT(val[u] * scale);
       }
     }
   }
@@ -490,12 +492,13 @@ __device__ __forceinline__ void hess_blocks(const World<NT, HT, NS>& w, const He
   }
 }
 
-// H <- A + J^T G J + diag for the warp's blocks from its accumulators.
+// H <- scale (A + J^T G J + diag) for the warp's blocks from its accumulators.
 template <int NT, typename HT, int NS, int Q0, int Q1>
 __device__ __forceinline__ void hess_store(const World<NT, HT, NS>& w, const HessBlocks<Q0, Q1>& blk,
                                            double diag_shift, const double (&acc)[Q0 + Q1][2]) {
   const int lane = threadIdx.x & 31, g = lane >> 2, l4 = lane & 3;
   const int n = w.dofs(), ldH = w.ldH();
+  const double scale = *w.scale;
 #pragma unroll
   for (int q = 0; q < Q0 + Q1; ++q) {
     const int i = 8 * blk.i[q] + g, j = 8 * (q < Q0 ? blk.j0 : blk.j1) + 2 * l4;
@@ -503,8 +506,8 @@ __device__ __forceinline__ void hess_store(const World<NT, HT, NS>& w, const Hes
       const double* Ai = w.A + i * n + j;
       HT* Hi = w.H + i * ldH + j;
       const double hd = w.V(V_HDIAG)[i] + diag_shift;
-      Hi[0] = HT(__ldg(Ai) + acc[q][0] + (i == j ? hd : 0.0));
-      if (j + 1 <= i) Hi[1] = HT(__ldg(Ai + 1) + acc[q][1] + (i == j + 1 ? hd : 0.0));
+      Hi[0] = HT((__ldg(Ai) + acc[q][0] + (i == j ? hd : 0.0)) * scale);
+      if (j + 1 <= i) Hi[1] = HT((__ldg(Ai + 1) + acc[q][1] + (i == j + 1 ? hd : 0.0)) * scale);
     }
   }
 }
@@ -603,7 +606,7 @@ template <int NT, typename HT, int NS>
 __device__ void solve_warp(const World<NT, HT, NS>& w, int rhs_slot, int out_slot, int warp) {
   if ((threadIdx.x >> 5) == warp) {
     const HT* dinv = reinterpret_cast<const HT*>(w.V(V_DINV));
-    const bool ok = ldlt_pivots_ok_warp<HT>(w.H, w.dofs(), w.ldH());
+    const bool ok = ldlt_pivots_ok_warp<HT>(dinv, w.dofs());
     ldlt_solve_warp<HT>(w.H, w.dofs(), w.ldH(), dinv, w.V(rhs_slot), w.V(out_slot), true, ok);
   }
 }
@@ -631,6 +634,19 @@ __device__ __forceinline__ void line_coefficients(const World<NT, HT, NS>& w, do
   }
 }
 
+// The powers of two by which a world's H is scaled, right-hand sides alike (so
+// that directions are the same bits): 1, and where diag(A) comes near an end
+// of the factor's type, away from it, so that pivots stay within pivot_recip's
+// range.  (Always multiplied with: eight products a thread and iteration.)
+template <typename HT>
+struct WorldScale {
+  static constexpr bool k64 = sizeof(HT) == 8;
+  // 2^+-900 and 2^+-64, or 2^+-100 and 2^+-8
+  static constexpr double kBig = k64 ? 8.452712498170644e270 : 1.2676506002282294e30;
+  static constexpr double kUp = k64 ? 1.8446744073709552e19 : 256.0;
+  static constexpr double kSmall = 1.0 / kBig, kDown = 1.0 / kUp;
+};
+
 constexpr int kMixed = -1;  // NS of the kernel that holds every size class's code
 template <int NS> struct LdltBlocks { static constexpr int kCount = 1; static constexpr int kW[1] = {4}; };
 template <> struct LdltBlocks<35> { static constexpr int kCount = 2; static constexpr int kW[2] = {5, 4}; };
@@ -644,7 +660,8 @@ template <> struct LdltBlocks<6> { static constexpr int kCount = 1; static const
 // hold more DOFs than the world has.
 template <int NT, typename HT, int NS, int LSV, int LB>
 __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& L, unsigned char* smem, double* red,
-                                            unsigned long long& s_partmask, int& s_factor_ok, const int e,
+                                            unsigned long long& s_partmask, double& s_scale, int& s_factor_ok,
+                                            const int e,
                                             const int n_max, const int n_rt, const bool use_guess) {
   const int tid = threadIdx.x;
   const int C = P.p.max_contacts;
@@ -663,6 +680,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
                       reinterpret_cast<int*>(fx + F.off_flags),
                       reinterpret_cast<const uint16_t*>(smem),
                       red,
+                      &s_scale,
                       &s_factor_ok,
                       n,
                       0};
@@ -721,6 +739,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
         }
         w.V(V_V)[i] = v;
         double d = __ldg(w.A + (size_t)i * n + i);
+        if (d > 0.0 && d < WorldScale<HT>::kSmall) s_scale = WorldScale<HT>::kUp;  // (1 before; any thread)
         if (d < 1.0e-12 || !isfinite(d)) d = 1.0e-12;
         w.V(V_ADIAG)[i] = d;
         w.V(V_DSCALE)[i] = 1.0 / sqrt(d);
@@ -835,6 +854,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
     const int model = (w.flags[i] & (kFlagPd | kFlagLo | kFlagUp)) ? 1 : 0;
     any_model_term |= model;
     if (model || ((s_partmask >> i) & 1ull)) w.flags[i] |= kFlagPart;
+    if (w.V(V_ADIAG)[i] > WorldScale<HT>::kBig) s_scale = WorldScale<HT>::kDown;
   }
   const int model_terms = __syncthreads_or(any_model_term);
   const bool unconstrained = (count == 0) && !model_terms;
@@ -933,7 +953,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
                 const double* Lg = P.p.dynamics_factor + (size_t)e * n_max * n_max;
                 load_lower<NT, HT, NS>(w, Lg);
 #pragma unroll 1
-                for (int i = tid; i < n; i += NT) dinv[i] = fast_recip(HT(__ldg(Lg + (size_t)i * n + i)));
+                for (int i = tid; i < n; i += NT) dinv[i] = fast_recip(HT(__ldg(Lg + (size_t)i * n + i) * s_scale));
               } else {
                 load_lower<NT, HT, NS>(w, w.A);
                 __syncthreads();
@@ -971,7 +991,7 @@ __device__ __forceinline__ void solve_world(const SolveParams& P, const Layout& 
                     const double* Jc = w.J + (size_t)(3 * c) * ldj;
                     acc += Jc[i] * g[3 * c] + Jc[ldj + i] * g[3 * c + 1] + Jc[2 * ldj + i] * g[3 * c + 2];
                   }
-                  w.V(kk == 0 ? V_GRAD : V_DP)[i] = -acc;  // the solves give -H^-1 rhs
+                  w.V(kk == 0 ? V_GRAD : V_DP)[i] = -acc * *w.scale;  // the solves give -H^-1 rhs
                 }
               }
               __syncthreads();
@@ -1114,6 +1134,7 @@ __global__ void __launch_bounds__(NT, MINB) contact_solve_kernel(const SolvePara
   __shared__ double red[kRedSize * (NT / 32)];
   __shared__ int s_next;
   __shared__ unsigned long long s_partmask;
+  __shared__ double s_scale;
   __shared__ int s_factor_ok;
   const int tid = threadIdx.x;
   // n_max: the DOF slots of a world in the arrays; a world's own DOF count may
@@ -1139,7 +1160,10 @@ __global__ void __launch_bounds__(NT, MINB) contact_solve_kernel(const SolvePara
     if (ticket >= P.p.num_envs) break;
     const int e = P.p.world_order ? P.p.world_order[ticket] : ticket;
     __syncthreads();
-    if (tid == 0) s_next = atomicAdd(P.queue, 1);
+    if (tid == 0) {
+      s_next = atomicAdd(P.queue, 1);
+      s_scale = 1.0;
+    }
     __syncthreads();
     if (e < 0 || e >= P.p.num_envs) continue;
     const int n_world = dofs_of(e);
@@ -1189,7 +1213,7 @@ __global__ void __launch_bounds__(NT, MINB) contact_solve_kernel(const SolvePara
       // each world's own DOF count: the specialised code of its size class
 #define SAPB_CLASS(N)                                                                                              \
   case N:                                                                                                          \
-    solve_world<NT, HT, N, LSV, LdltBlocks<N>::kW[0]>(P, L, smem, red, s_partmask, s_factor_ok, e, n_max, N, use_guess); \
+    solve_world<NT, HT, N, LSV, LdltBlocks<N>::kW[0]>(P, L, smem, red, s_partmask, s_scale, s_factor_ok, e, n_max, N, use_guess); \
     break;
       switch (n_world) {
         SAPB_CLASS(35)
@@ -1197,11 +1221,11 @@ __global__ void __launch_bounds__(NT, MINB) contact_solve_kernel(const SolvePara
         SAPB_CLASS(13)
         SAPB_CLASS(6)
         default:
-          solve_world<NT, HT, 0, LSV, LB>(P, L, smem, red, s_partmask, s_factor_ok, e, n_max, n_world, use_guess);
+          solve_world<NT, HT, 0, LSV, LB>(P, L, smem, red, s_partmask, s_scale, s_factor_ok, e, n_max, n_world, use_guess);
       }
 #undef SAPB_CLASS
     } else {
-      solve_world<NT, HT, NS, LSV, LB>(P, L, smem, red, s_partmask, s_factor_ok, e, n_max, n_world, use_guess);
+      solve_world<NT, HT, NS, LSV, LB>(P, L, smem, red, s_partmask, s_scale, s_factor_ok, e, n_max, n_world, use_guess);
     }
   }
 }

@@ -29,10 +29,15 @@ __device__ __forceinline__ void build_triangle_list(uint16_t* tri, int n, int nr
 }
 
 // Pivot reciprocal of the factorization: Newton-Raphson steps from the
-// hardware's approximation (two in FP64, one in FP32), without a range check:
-// a pivot that is not positive and finite, or beyond the reciprocal's range,
-// gives one that is not, and is reported by it (ldlt_backward_warp,
-// ldlt_pivots_ok_warp).
+// hardware's approximation (two in FP64, one in FP32), without a range check.
+// Of a pivot that is not positive and finite, or outside the approximation's
+// range (subnormal, or beyond 2^126 in FP32 and 2^1022 in FP64), the result is
+// no positive normal number: such pivots are kept away from it (the dense solve
+// scales that world's H, WorldScale; the tree-blocked solve factors that block
+// again with divisions) or reported like bad ones (the free motion's in FP64,
+// whose velocity is then NaN).  A guard on each pivot is on the serial chain; a
+// check of every block's reciprocals with divisions behind it cost 2 % of the
+// dense solves and the free motion.
 __device__ __forceinline__ double pivot_recip(double d) {
   double x;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(x) : "d"(d));
@@ -43,6 +48,17 @@ __device__ __forceinline__ float pivot_recip(float d) {
   float x;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(x) : "f"(d));
   return fmaf(x, fmaf(-d, x, 1.0f), x);
+}
+
+__device__ __forceinline__ bool positive_normal(double r) {
+  return (unsigned)(__double2hiint(r) - 0x00100000) < 0x7fe00000u;
+}
+__device__ __forceinline__ bool positive_normal(float r) {
+  return (unsigned)(__float_as_int(r) - 0x00800000) < 0x7f000000u;
+}
+template <bool DIVIDE, typename T>
+__device__ __forceinline__ T pivot(T d) {
+  return DIVIDE ? T(1) / d : pivot_recip(d);
 }
 
 // Values of S (the scaled panel) per row: B rounded up so that rows are
@@ -274,10 +290,7 @@ __device__ void ldlt_solve_blocked(const T* H, int n, int ldH, const T* dinv, X*
   const int tid = threadIdx.x;
   constexpr int B = sizeof(T) == 4 ? 8 : 6;
   bool ok = true;
-  for (int k = 0; k < n; ++k) {
-    const T d = H[(size_t)k * ldH + k];
-    if (!(d > T(0)) || !isfinite(double(d))) ok = false;
-  }
+  for (int k = 0; k < n; ++k) ok = ok && dinv[k] > T(0) && dinv[k] < T(INFINITY);
   const T sgn = neg ? T(-1) : T(1);
   // forward
   for (int K = 0; K < n; K += B) {
@@ -388,16 +401,13 @@ __device__ __forceinline__ void ldlt_solve_warp(const T* H, int n, int ldH, cons
   if (lane + 32 < n) x[lane + 32] = ok ? double(z1) : nanv;
 }
 
-// Whether every pivot of a stored LDL^T is positive and finite (the warp's
-// lanes check two each), returned to every lane.
+// Whether every pivot of a stored LDL^T is positive and finite by its
+// reciprocal (the warp's lanes check two each), returned to every lane.
 template <typename T>
-__device__ bool ldlt_pivots_ok_warp(const T* H, int n, int ldH) {
+__device__ __forceinline__ bool ldlt_pivots_ok_warp(const T* dinv, int n) {
   const int lane = threadIdx.x & 31;
   bool ok = true;
-  for (int k = lane; k < n; k += 32) {
-    const T d = H[(size_t)k * ldH + k];
-    if (!(d > T(0)) || !isfinite(double(d))) ok = false;
-  }
+  for (int k = lane; k < n; k += 32) ok = ok && dinv[k] > T(0) && dinv[k] < T(INFINITY);
   return __all_sync(0xffffffffu, ok);
 }
 

@@ -760,7 +760,7 @@ __global__ void __launch_bounds__(kPrepNT, VS ? 5 : 6) prepare_world_kernel(cons
   auto POSE_P = [&](int b) { return v3(pose[8 * b], pose[8 * b + 1], pose[8 * b + 2]); };
   auto POSE_Q = [&](int b) { return Q4{pose[8 * b + 3], pose[8 * b + 4], pose[8 * b + 5], pose[8 * b + 6]}; };  // unit
   if (split && tid < 32) {
-    ldlt_solve_warp<double>(H, n, n, dinv, tau, vdot, false, ldlt_pivots_ok_warp<double>(H, n, n));
+    ldlt_solve_warp<double>(H, n, n, dinv, tau, vdot, false, ldlt_pivots_ok_warp<double>(dinv, n));
   } else {
   const int wt = split ? tid - 32 : tid;                // worker thread index
   const int wn = split ? kPrepNT - 32 : kPrepNT;        // worker threads
@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(kPrepNT, VS ? 5 : 6) prepare_world_kernel(cons
         jg[i] = r;
       }
       __syncwarp();
-      ldlt_solve_warp<double>(H, n, n, dinv, jg, z, false, ldlt_pivots_ok_warp<double>(H, n, n));
+      ldlt_solve_warp<double>(H, n, n, dinv, jg, z, false, ldlt_pivots_ok_warp<double>(dinv, n));
       __syncwarp();
       for (int i = tid; i < n; i += 32)
         P.out.v_start[vs0 + i] = P.in.joint_qd[d0 + i] + P.in.dt[e] * vdot[i] + z[i];

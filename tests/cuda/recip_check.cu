@@ -1,4 +1,4 @@
-// Checks sapb::fast_recip (Newton-Raphson from an FP32 seed) against the
+// Checks sapb::fast_recip (Newton-Raphson from the hardware's approximation) against the
 // IEEE division 1.0/d on the GPU: prints the largest error in ulps.
 #include <cstdio>
 #include <cstdlib>
@@ -29,7 +29,7 @@ int main() {
   srand(12345);
   for (int i = 0; i < n; ++i) {
     double u = (double)rand() / RAND_MAX, s = (rand() & 1) ? 1.0 : -1.0;
-    h[i] = s * pow(10.0, -35.0 + 70.0 * u);  // spans the fast range and both fallbacks
+    h[i] = s * pow(10.0, -35.0 + 70.0 * u);  // within the range that takes no division
   }
   double *dh, *df, *dr;
   cudaMalloc(&dh, n * 8);
