@@ -11,10 +11,11 @@ solve reaches); and a runtime-size kernel with 256 threads per world, which
 pays where shared memory leaves one CTA per SM.  The tuner times every
 (k, b, threads) on the caller's own first solve (CUDA events, best of a few
 runs each) and keeps the fastest in a table keyed by (DOFs per world,
-contact-slot bucket, precision, line search, GPU name, SM count), which it
-can persist as JSON.  The default shape (the
-occupancy bound, the first width) is kept unless another beats it by more
-than a margin.
+contact-slot bucket, precision, line search, GPU name, SM count, for uneven
+batches their launch plan), which it can persist as JSON.  The default shape
+-- what an untuned launch does: the occupancy bound and the first width of a
+specialised kernel, else (0, 0, 0), the dispatch's own choice -- is kept
+unless another beats it by more than a margin.
 """
 
 from __future__ import annotations
@@ -32,11 +33,16 @@ def contact_bucket(max_contacts: int) -> int:
     return b
 
 
+# Raised when the kernels change so that a choice timed on earlier ones may no
+# longer be the fastest: entries of other values are timed again.
+KERNELS = 2
+
+
 def tuning_key(dof_per_env: int, max_contacts: int, precision: str, line_search: str, gpu_name: str,
-               sm_count: int) -> str:
+               sm_count: int, plan: str = "") -> str:
     gpu = "".join(ch if ch.isalnum() else "_" for ch in str(gpu_name)).strip("_")
     return (f"n{int(dof_per_env)}-c{contact_bucket(max_contacts)}-{precision}-{line_search}-{gpu}-"
-            f"{int(sm_count)}sm")
+            f"{int(sm_count)}sm" + (f"-{plan}" if plan else ""))
 
 
 def _label(shape) -> str:
@@ -69,21 +75,22 @@ class SolveAutotuner:
 
     def lookup(self, key: str):
         entry = self.table.get(key)
-        if entry is None:
+        if entry is None or entry.get("kernels") != KERNELS:
             return None
         return _shape(entry["choice"]) if "choice" in entry else int(entry["ctas_per_sm"])
 
     def tune(self, key: str, candidates: list, time_ms: Callable, default=None):
         """The cached choice for `key`, else the candidate with the least time,
-        recorded with every candidate's time.  The default (given, or for
-        plain ints the largest: the occupancy bound, the launch without
-        tuning) is kept unless another beats it by more than `margin` (a
+        recorded with every candidate's time.  The default (given -- it may be
+        (0, 0, 0), the launch without tuning -- or for plain ints the largest:
+        the occupancy bound) is kept unless another beats it by more than `margin` (a
         short sample decides)."""
         known = self.lookup(key)
         if known is not None:
             return known
         cands = [_shape(c) for c in candidates]
-        cands = [c for c in dict.fromkeys(cands) if (min(c) if isinstance(c, tuple) else c) >= 1]
+        keep = None if default is None else _shape(default)
+        cands = [c for c in dict.fromkeys(cands) if c == keep or (min(c) if isinstance(c, tuple) else c) >= 1]
         if not cands:
             raise ValueError("no candidate launch shape")
         if default is None:
@@ -97,7 +104,7 @@ class SolveAutotuner:
             best = default
         entry = {"choice": list(best) if isinstance(best, tuple) else best,
                  "ctas_per_sm": best[0] if isinstance(best, tuple) else best,
-                 "ms": {_label(c): times[c] for c in cands}}
+                 "ms": {_label(c): times[c] for c in cands}, "kernels": KERNELS}
         self.table[key] = entry
         self.save()
         return best

@@ -693,11 +693,11 @@ class SapContactSolve:
         """(resident CTAs per SM, LDL^T block width, threads per CTA) for this
         problem: (0, 0, 0) -- the occupancy bound, the default width and
         kernel -- without an autotuner; with one, its choice for the
-        problem's key among every CTA count up to the bound and every width
-        the kernel is built with, and every CTA count of the 256-thread
-        runtime-size kernel, timed here on this very problem the first time
-        the key is seen
-        (never while a graph is being captured: then the defaults).  The solve
+        problem's key among that launch, every CTA count up to the bound and
+        every width the kernel is built with, and every CTA count of the
+        256-thread runtime-size kernel, timed here on this very problem the
+        first time the key is seen (never while a graph is being captured:
+        then the defaults).  The solve
         writes its start back into the warm-start guess `guess` (and the
         guess may be the output velocity itself), so the guess is saved
         before the timed solves and restored before each of them and after:
@@ -711,8 +711,13 @@ class SapContactSolve:
         if self._device_props is None:
             self._device_props = torch.cuda.get_device_properties(v.device)
         props = self._device_props
+        # uneven batches run in one launch, beyond 16 worlds per SM in one per
+        # size class (sapb_contact_solve.cu)
+        plan = ""
+        if P.dof_count:
+            plan = "classes" if v.W > 16 * props.multi_processor_count else "mixed"
         key = tuning_key(v.n, P.max_contacts, "fp32" if fp32 else "fp64", variant, props.name,
-                         props.multi_processor_count)
+                         props.multi_processor_count, plan)
         known = self.autotuner.lookup(key)
         if known is not None:
             known = known if isinstance(known, tuple) else (known,)
@@ -744,17 +749,24 @@ class SapContactSolve:
             e1.synchronize()
             return e0.elapsed_time(e1)
 
-        cands = [(k, int(widths[b]), 128) for b in range(nw) for k in range(1, occ + 1)]
+        gw = (ctypes.c_int32 * 8)()
+        ngw = lib.sapb_contact_solve_ldlt_blocks(1, gw, 8)  # the runtime-size kernel's widths
+        # The untuned launch is the specialised kernel at its occupancy bound,
+        # or else the dispatch's choice: of 128 and 256 threads for a count
+        # without a specialised kernel, of each size class's own occupancy for
+        # an uneven batch (whose largest world's would cap the others')
+        specialised = list(widths)[:nw] != list(gw)[:ngw]
+        default = (occ, int(widths[0]), 128) if specialised and not P.dof_count else (0, 0, 0)
+        cands = [] if default[0] else [default]
+        cands += [(k, int(widths[b]), 128) for b in range(nw) for k in range(1, occ + 1)]
         # the runtime-size kernel with eight warps per world (its default
         # width), where its shared memory fits
         occ_wide = int(lib.sapb_contact_solve_occupancy_threads(v.n, int(P.max_contacts),
                                                                 _abi.SAPB_FP32 if fp32 else _abi.SAPB_FP64,
                                                                 int(opts.line_search_variant), 256))
         if occ_wide >= 1:
-            gw = (ctypes.c_int32 * 8)()
-            lib.sapb_contact_solve_ldlt_blocks(1, gw, 8)  # the runtime-size kernel's widths
             cands += [(k, int(gw[0]), 256) for k in range(1, occ_wide + 1)]
-        chosen = self.autotuner.tune(key, cands, time_ms, default=(occ, int(widths[0]), 128))
+        chosen = self.autotuner.tune(key, cands, time_ms, default=default)
         if saved is not None:
             guess.copy_(saved)
         return chosen

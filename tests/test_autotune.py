@@ -45,3 +45,27 @@ def test_the_occupancy_bound_stays_within_the_margin():
     tuner = SolveAutotuner(margin=0.05)
     assert tuner.tune("s", [1, 2, 3, 4], {1: 2.0, 2: 1.0, 3: 0.99, 4: 1.03}.get) == 4
     assert tuner.tune("t", [1, 2, 3, 4], {1: 2.0, 2: 1.0, 3: 0.90, 4: 1.03}.get) == 3
+
+
+def test_the_untuned_launch_is_a_candidate_and_the_default():
+    tuner = SolveAutotuner()
+    cands = [(0, 0, 0), (1, 4, 128), (2, 4, 128)]
+    assert tuner.tune("s", cands, {(0, 0, 0): 1.02, (1, 4, 128): 2.0, (2, 4, 128): 1.0}.get, default=(0, 0, 0)) == \
+        (0, 0, 0)  # within the margin
+    assert tuner.lookup("s") == (0, 0, 0)
+    assert tuner.tune("t", cands, {(0, 0, 0): 1.1, (1, 4, 128): 2.0, (2, 4, 128): 1.0}.get, default=(0, 0, 0)) == \
+        (2, 4, 128)
+
+
+def test_keys_name_the_plan_of_an_uneven_batch():
+    args = (35, 32, "fp32", "armijo_decay", "NVIDIA B200", 148)
+    assert len({tuning_key(*args), tuning_key(*args, "mixed"), tuning_key(*args, "classes")}) == 3
+
+
+def test_choices_timed_on_other_kernels_are_timed_again(tmp_path):
+    path = tmp_path / "old.json"
+    path.write_text(json.dumps({"s": {"choice": [1, 4, 128], "ctas_per_sm": 1, "ms": {"1,4,128": 1.0}}}))
+    tuner = SolveAutotuner(path)
+    assert tuner.lookup("s") is None
+    assert tuner.tune("s", [(1, 4, 128), (2, 4, 128)], lambda c: 1.0 / c[0], default=(1, 4, 128)) == (2, 4, 128)
+    assert SolveAutotuner(path).lookup("s") == (2, 4, 128)

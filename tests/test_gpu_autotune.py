@@ -174,3 +174,24 @@ def test_wide_kernel_matches_the_oracle(cuda_device, oracle, kind):
         want = ref["v"].reshape(-1, n)
         err = np.abs(got - want).max(1) / np.maximum(np.abs(want).max(1), 1e-30)
         assert np.quantile(err, 0.98) <= 1e-6 and err.max() <= 1e-4, (kind, prec, err.max())
+
+
+@pytest.mark.parametrize("worlds_per_kind, plan", [(8, "mixed"), (800, "classes")])
+def test_uneven_batches_keep_the_untuned_launch_as_the_default(cuda_device, tmp_path, worlds_per_kind, plan):
+    """The untuned launch, in which each size class has its own occupancy, is
+    timed with the others and stays unless it is beaten by more than the margin."""
+    path = tmp_path / "uneven.json"
+    model, state, control, contacts, _ = models.mixed_rollout_scene(worlds_per_kind, 87, cuda_device)
+    solver = SolverSAP(model, max_rigid_contact=32, contact_preset_variant="drake", hessian_precision="fp32",
+                       autotune=str(path))
+    out = SapState(joint_q=state.joint_q.clone(), joint_qd=state.joint_qd.clone(), body_q=state.body_q.clone(),
+                   body_f=state.body_f.clone())
+    solver.step(state, out, control, contacts, 2e-3)
+    torch.cuda.synchronize()
+    (key, entry), = json.loads(path.read_text()).items()
+    assert key.endswith("-" + plan) and "0,0,0" in entry["ms"]
+    best = min(entry["ms"].values())
+    if entry["choice"] == [0, 0, 0]:
+        assert entry["ms"]["0,0,0"] <= 1.03 * best * (1 + 1e-12)
+    else:
+        assert best * 1.03 < entry["ms"]["0,0,0"]
