@@ -686,13 +686,10 @@ def main():
                                                                       opts.line_search_variant, 256))
         gw = (__import__("ctypes").c_int32 * 8)()
         _load_lib().sapb_contact_solve_ldlt_blocks(1, gw, 8)
-        # the untuned launch: of an uneven batch each size class's own occupancy
-        default = (0, 0, 0) if "dof_count" in tt else (occ, int(wl[0]), 128)
-        cands = [] if default[0] else [default]
-        cands += [(k, int(wl[w]), 128) for w in range(nw) for k in range(1, occ + 1)]
+        cands = [(k, int(wl[w]), 128) for w in range(nw) for k in range(1, occ + 1)]
         cands += [(k, int(gw[0]), 256) for k in range(1, occ_w + 1)]
         tuner = SolveAutotuner(repeats=5)
-        chosen = tuner.tune(label, cands, time_ms, default=default)
+        chosen = tuner.tune(label, cands, time_ms, default=(occ, int(wl[0]), 128))
         opts.ctas_per_sm, opts.ldlt_block, opts.threads_per_cta = 0, 0, 0
         tuned[label] = {"occupancy": occ, "occupancy_256_threads": occ_w, "ldlt_blocks": [int(wl[w]) for w in range(nw)],
                         "chosen": list(chosen), "ms": tuner.table[label]["ms"]}
