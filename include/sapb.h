@@ -100,7 +100,8 @@ typedef struct sapb_solve_options {
   double line_search_relative_slop; /* 1000 * eps(fp64) */
   int32_t line_search_variant;    /* SAPB_LS_* ; solve() default monotone_decay */
   int32_t linear_solve_precision; /* SAPB_FP64 / SAPB_FP32: Newton-direction Cholesky */
-  int32_t hessian_precision;      /* SAPB_FP64 / SAPB_FP32: J^T G J assembly */
+  int32_t hessian_precision;      /* SAPB_FP64 / SAPB_FP32: H = A + J^T G J as it is factored; the dense solve
+                                   * sums it in FP64 and rounds once, the tree-blocked solve sums in this type */
   int32_t cubic_init;             /* exact_root cubic seed, sim/contact_solve.py:55-58 (1) */
   int32_t ctas_per_sm;            /* resident CTAs per SM of the persistent dense solve: 0 as many as fit
                                    * (sapb_contact_solve_occupancy), k at most k; results do not depend on it */

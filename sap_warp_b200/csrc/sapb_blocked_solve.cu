@@ -53,7 +53,7 @@ int32_t blocked_solve_launch(const sapb_blocked_problem* p, const sapb_solve_opt
   int threads = o->threads_per_cta;
   if (threads != 128 && threads != 256) {
     const int n = p->trees_per_env * p->tree_dofs;
-    threads = n <= 128 ? 128 : (p->tree_dofs == 6 && n >= 360 ? 512 : 256);
+    threads = n <= 128 ? 128 : (p->tree_dofs == 6 && n >= blk::kBWideDofs ? blk::kBWideThreads : 256);
   }
   cudaError_t err;
   switch (p->tree_dofs) {

@@ -49,6 +49,13 @@ namespace blk {
 
 constexpr int kBMaxTrees = 64;
 
+// Worlds of free bodies of this many DOFs and more run this many threads, with
+// the reductions' scratch in the place of the block solves' (zd), which
+// therefore has to hold it in FP32 too.
+constexpr int kBWideThreads = 512, kBWideDofs = 360;
+static_assert(kBWideDofs * sizeof(float) >= 2 * kRedBatch * (kBWideThreads / 32) * sizeof(double),
+              "zd holds the reductions' scratch");
+
 struct BlockedParams {
   sapb_blocked_problem p;
   sapb_dof_terms dof;  // the drive / limit terms (all zero without)
@@ -802,10 +809,10 @@ __device__ bool bsymbolic(const BWorld<NT, HT, NB>& w, int cap) {
 template <int NT, typename HT, int NB, int LSV>
 __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParams P) {
   extern __shared__ __align__(16) unsigned char smem[];
-  // the reductions' scratch; with 512 threads in the place of the block solves'
-  // (not in use beside them), where the static arrays leave no room
+  // the reductions' scratch; with kBWideThreads in the place of the block
+  // solves' (not in use beside them), where the static arrays leave no room
   constexpr int kRed = 2 * kRedBatch * (NT / 32);
-  __shared__ double red_own[NT < 512 ? kRed : 1];
+  __shared__ double red_own[NT < kBWideThreads ? kRed : 1];
   __shared__ int s_next;
   __shared__ int16_t s_tstart[kBMaxTrees], s_tcount[kBMaxTrees];  // world DOFs: at most 64 x 12
   __shared__ int s_bad_layout;
@@ -862,7 +869,7 @@ __global__ void __launch_bounds__(NT, 1) blocked_solve_kernel(const BlockedParam
     w.vec = reinterpret_cast<double*>(smem + L.off_vec);
     w.con = reinterpret_cast<double*>(smem + L.off_con);
     w.flags = reinterpret_cast<int*>(smem + L.off_flags);
-    w.red = NT < 512 ? red_own : reinterpret_cast<double*>(smem + L.off_zd);
+    w.red = NT < kBWideThreads ? red_own : reinterpret_cast<double*>(smem + L.off_zd);
     w.A = P.p.tree_mass + (size_t)e * T * NB * NB;
     w.J = P.p.jacobian + (size_t)e * C * 3 * 2 * NB;
     w.tree = reinterpret_cast<const int8_t*>(smem + L.off_tree);
@@ -1284,15 +1291,17 @@ cudaError_t launch_blocked_nt(const BlockedParams& P, cudaStream_t stream) {
 }
 
 // One block size's kernels (both Hessian precisions, 128 or 256 threads per
-// world, also 512 for free bodies, every line search), instantiated in a translation unit of its own
-// (sapb_blocked_nb{6,7,12}.cu) so they compile in parallel.
+// world, also 512 for free bodies, every line search), instantiated in a
+// translation unit of its own (sapb_blocked_nb{6,7,12}.cu) so they compile in
+// parallel.
 template <int NB>
 cudaError_t launch_blocked(const BlockedParams& P, bool fp32, int threads, cudaStream_t stream) {
   if (threads == 128)
     return fp32 ? launch_blocked_nt<128, float, NB>(P, stream) : launch_blocked_nt<128, double, NB>(P, stream);
   if constexpr (NB == 6)
-    if (threads == 512)
-      return fp32 ? launch_blocked_nt<512, float, NB>(P, stream) : launch_blocked_nt<512, double, NB>(P, stream);
+    if (threads == kBWideThreads && P.p.trees_per_env * NB >= kBWideDofs)
+      return fp32 ? launch_blocked_nt<kBWideThreads, float, NB>(P, stream)
+                  : launch_blocked_nt<kBWideThreads, double, NB>(P, stream);
   return fp32 ? launch_blocked_nt<256, float, NB>(P, stream) : launch_blocked_nt<256, double, NB>(P, stream);
 }
 extern template cudaError_t launch_blocked<6>(const BlockedParams&, bool, int, cudaStream_t);

@@ -120,9 +120,9 @@ int32_t contact_solve_launch(const sapb_contact_problem* p, const sapb_solve_opt
   P.use_guess_flag_ptr_valid = (p->v_guess && p->v_guess_active) ? 1 : 0;
   P.queue = reinterpret_cast<int32_t*>(workspace);
   if (p->num_envs == 0) return SAPB_OK;
-  // If either the Hessian or the linear-solve precision is FP32, both the
-  // J^T G J assembly and the LDL^T factorization run in FP32; the gradient,
-  // costs, line search and convergence test stay FP64 in every variant.
+  // If either the Hessian or the linear-solve precision is FP32, H is rounded
+  // to FP32 and its LDL^T factorization runs in it; the sums of J^T G J, the
+  // gradient, costs, line search and convergence test are FP64 in every variant.
   const bool fp32 = o->hessian_precision == SAPB_FP32 || o->linear_solve_precision == SAPB_FP32;
   const size_t smem =
       contact_solve_smem_bytes(p->dof_per_env, p->max_contacts, fp32 ? SAPB_FP32 : SAPB_FP64, o->threads_per_cta);

@@ -5,15 +5,16 @@
 // the world's contact Jacobian J in shared memory once, and runs prepare
 // (:4285-4429), the Newton loop (:5474-5655) and the chosen line search
 // (:2207-3175) on chip.  The dynamics matrix A is read through L1 (it is the
-// only per-world array re-read from outside shared memory; 3-4 passes per
-// Newton iteration hit L1/L2).  Per line-search trial the kernel touches
+// only per-world array re-read from outside shared memory: twice a Newton
+// iteration, for A dv and for the Hessian, from L1/L2).  Per line-search trial the kernel touches
 // O(contacts + DOFs) data because the contact velocity along the search line
 // is vc + alpha * (J dv) (vc is linear in v); the reference issues ~35
 // launches per Newton iteration and re-reads A and J on every trial.
 //
-// Precision: the gradient, costs, line search, velocity update and the
-// convergence test are FP64.  The Hessian H = A + J^T G J + diag and its LDL^T
-// factorization run in HT (double, or float for the mixed path).
+// Precision: the gradient, costs, line search, velocity update, the convergence
+// test and the sums of the Hessian H = A + J^T G J + diag are FP64.  H is rounded
+// once to HT (double, or float for the mixed path), in which its LDL^T
+// factorization runs.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -1297,9 +1298,10 @@ inline cudaError_t launch_solve_ns(const SolveParams& P, bool fp32, cudaStream_t
 }
 
 // The runtime-size kernel with 256 threads (eight warps) per world, the
-// default LDL^T width: for worlds whose shared memory leaves one or two CTAs
-// per SM (sapb_solve_options.threads_per_cta = 256), instantiated in
-// sapb_solve_nwide_f32.cu / _f64.cu.
+// default LDL^T width: on request (sapb_solve_options.threads_per_cta = 256), and
+// by itself for worlds without a specialised kernel whose shared memory leaves
+// one CTA per SM (solve_dispatch); instantiated in sapb_solve_nwide_f32.cu /
+// _f64.cu.
 template <bool FP32>
 cudaError_t launch_solve_wide(const SolveParams& P, cudaStream_t stream, int* blocks_out) {
   using HT = typename std::conditional<FP32, float, double>::type;
