@@ -183,10 +183,14 @@ class _ModelView:
         is the ground)."""
         m = self.model
         J, B = int(m.joint_count), int(m.body_count)
-        parent = m.joint_parent.cpu().numpy().astype(np.int64)[:J]
-        child = m.joint_child.cpu().numpy().astype(np.int64)[:J]
-        live = (parent >= 0) & (parent < B) & (child >= 0) & (child < B)
-        joint, parent, child = np.flatnonzero(live), parent[live], child[live]
+        parent, child = m.joint_parent.cpu().numpy()[:J], m.joint_child.cpu().numpy()[:J]
+        joint = np.flatnonzero((parent >= 0) & (parent < B) & (child >= 0) & (child < B))
+        parent, child = parent[joint], child[joint]
+        # parents' joints all before their children's, as models are mostly laid out: no cycle
+        last = np.full(B, -1, np.int64)
+        last[child] = joint
+        if np.all(last[parent] < joint):
+            return
         if self.uneven:
             jworld = np.searchsorted(self.world_offsets["joint"], joint, side="right")
             pworld, cworld = (np.searchsorted(self.world_offsets["body"], b, side="right") for b in (parent, child))
