@@ -3,7 +3,8 @@ the FP32 factor (its own panel strides and instantiations) and with
 monotone_decay, worlds that fill an SM with the FP32 factor, the box counts
 around the 512-thread launch in both precisions, and the launches per size class
 of a large uneven batch with candidate starts, a kept factor, a guess, drives,
-limits and worlds without contacts, against the same worlds in small batches.
+limits and worlds without contacts, against the same worlds in small batches;
+and a tree-blocked candidate start that is rejected.
 
 Tolerances: FP32 directions and monotone_decay (here with the other searches'
 cost tolerance) may take other paths than the oracle, so up to half of a batch may be loose in
@@ -18,7 +19,8 @@ import pytest
 import torch
 
 from sap_warp_b200 import scenes
-from sap_warp_b200._solve import ContactSolveBuffers, DofTermArrays, contact_solve, make_options
+from sap_warp_b200._solve import (ContactSolveBuffers, DofTermArrays, blocked_contact_solve,
+                                  blocked_problem_to_device, contact_solve, make_options)
 from tests.test_gpu_blocked import run_blocked
 from tests.test_gpu_contact_solve import assert_parity, run_gpu
 from tests.test_gpu_far_start import check_reported
@@ -148,3 +150,24 @@ def test_class_launches_with_every_start_and_term(cuda_device, precision, kind):
             assert torch.equal(getattr(whole, name)[sl], getattr(part, name)), name
         live = torch.arange(C, device=cuda_device)[None] < arrays["contact_count"][sl][:, None]
         assert not bool(part.contact_gamma[~live].any()) and not bool(whole.contact_gamma[sl][~live].any())
+
+
+@pytest.mark.parametrize("boxes", [8, 30, 63])
+@pytest.mark.parametrize("threads", [0, 128, 256])
+def test_rejected_tree_blocked_candidate_leaves_the_plain_start(cuda_device, boxes, threads):
+    """Starting impulses far too large are evaluated and rejected: the solve
+    goes on from the plain start, which other threads save than overwrite, and
+    gives the bits of a solve without candidate."""
+    bp = scenes.box_stack_problem(24, seed=500 + boxes, boxes=boxes)
+    t = blocked_problem_to_device(bp, cuda_device)
+    g0 = torch.full((bp.num_envs, bp.max_contacts, 3), 1.0e3, dtype=torch.float64, device=cuda_device)
+    out = []
+    for gamma0 in (None, g0):
+        buf = ContactSolveBuffers(bp.num_envs, bp.dof_per_env, bp.max_contacts, cuda_device)
+        blocked_contact_solve(buffers=buf, options=make_options("armijo_decay", threads_per_cta=threads),
+                              trees_per_env=bp.trees_per_env, tree_dofs=bp.tree_dofs, gamma0=gamma0, **t)
+        torch.cuda.synchronize()
+        out.append(buf)
+    assert not bool(out[1].warm_start_accepted.any())
+    for name in ("v", "contact_gamma", "newton_iterations", "status"):
+        assert torch.equal(getattr(out[0], name), getattr(out[1], name)), name
